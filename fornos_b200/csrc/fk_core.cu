@@ -434,10 +434,13 @@ static int scene_create(fk_ctx* ctx, const fk_bvh_node* nodes, uint32_t nn, cons
     if (e != cudaSuccess) rc = fk_cuda_fail(ctx, e, "pair_boxes_kernel");
     else ++ctx->launches;
   }
+  if (rc == FK_OK)
+    rc = fk::ensure_tri_path(ctx, s, s->tree_wide[FK_TREE_SAH] ? FK_TREE_SAH : FK_TREE_REFERENCE);
   if (rc == FK_OK) {
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) rc = fk_cuda_fail(ctx, e, "scene upload sync");
   }
+  if (rc == FK_OK) s->tri_path = s->tree_path[FK_TREE_REFERENCE];
   if (rc != FK_OK) {
     ctx->scenes.insert(s);
     fk_scene_free(ctx, s);
@@ -541,7 +544,8 @@ int fk_scene_free(fk_ctx* ctx, fk_scene* s) {
   if (!ctx || !s || !ctx->scenes.count(s)) return fk_fail(ctx, FK_ERR_INVALID, "fk_scene_free: unknown scene");
   cudaStreamSynchronize(ctx->stream);
   void* ps[] = {s->node_lo,         s->node_hi,         s->node_jump, s->pos4,    s->nrm4,  s->tree_wide[0],
-                s->tree_wide[1],   s->tree_wide4[0],   s->tree_wide4[1], s->tri_rec, s->top, s->node_box};
+                s->tree_wide[1],   s->tree_wide4[0],   s->tree_wide4[1], s->tri_rec, s->top, s->node_box,
+                s->tree_path[0],   s->tree_path[1]};
   for (void* p : ps) fk_dev_free(ctx, p);
   ctx->scenes.erase(s);
   delete s;
@@ -556,8 +560,11 @@ int fk_scene_set_tree(fk_scene* s, int tree) {
   if (tree == FK_TREE_SAH && !s->tree_wide[FK_TREE_SAH] && !s->root_is_leaf)
     return fk_fail(ctx, FK_ERR_UNSUPPORTED, "fk_scene_set_tree: the rebuilt tree is deeper than the ordered traversal's 48");
   if (s->root_is_leaf) tree = FK_TREE_REFERENCE;  // a single leaf has no inner tree to rebuild
+  const int rc = fk::ensure_tri_path(ctx, s, tree);
+  if (rc != FK_OK) return rc;
   FK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // work queued on the previous tree is done
   s->tree = tree;
+  s->tri_path = s->tree_path[tree];
   s->wide = s->tree_wide[tree];
   s->wide4 = s->tree_wide4[tree];
   s->wide_count = s->tree_count[tree];

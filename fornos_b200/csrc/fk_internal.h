@@ -80,6 +80,10 @@ struct fk_scene {
   float4* wide4 = nullptr;
   uint32_t wide4_count = 0, depth4 = 0;
   float4* tri_rec = nullptr;
+  // Root-to-leaf path of each triangle's leaf in the 2-wide tree (SceneDev::tri_path): the active tree's, and
+  // both trees' once built.  Null for a single leaf or a tree deeper than kMaxOrderedDepth.
+  uint64_t* tri_path = nullptr;
+  uint64_t* tree_path[2] = {nullptr, nullptr};
   // The first inner records of the active 2-wide tree in breadth-first order
   // (fk_tuning.top_records), staged in shared memory by the ordered
   // traversal; a child ref >= wide_count names staged record ref - wide_count.
@@ -150,6 +154,9 @@ struct SceneDev {
   // read only for hits inside the distance range.
   const float4* __restrict__ rec;
   const float4* __restrict__ rec_bary;
+  // Per triangle, the way from the 2-wide tree's root record to the leaf that holds it: bit k is the child taken
+  // at level k (1: the second), ended by a set bit; 0 for a triangle that no leaf holds.  Null: no paths.
+  const uint64_t* __restrict__ tri_path;
   uint32_t node_count;
   uint32_t root_is_leaf;
   uint32_t corner_count;
@@ -285,6 +292,8 @@ int launch_gather(fk_ctx* ctx, const fk_scene* s, int kind, const float4* coords
                   uint32_t offset, uint32_t count, float* out);
 int launch_tangent_space(fk_ctx* ctx, const fk_texel_map* m, uint32_t offset, uint32_t count, float* io3);
 int launch_tri_records(fk_ctx* ctx, fk_scene* s);
+// fk_scene::tree_path[tree], built on first use (no-op where the tree has none).
+int ensure_tri_path(fk_ctx* ctx, fk_scene* s, int tree);
 // Fills box[2 i], box[2 i + 1] = lo[i], hi[i] for i < n on `stream`.
 cudaError_t pair_node_boxes(cudaStream_t stream, const float4* lo, const float4* hi, uint32_t n, float4* box);
 struct RasterTri;  // defined in fk_raster.cu

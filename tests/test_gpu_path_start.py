@@ -1,0 +1,54 @@
+"""Rays started at their own triangle's leaf (the 2-wide ordered traversal)
+against the skip-pointer walk: the occluder counts of AO do not depend on the
+order in which leaves are visited, so both are equal exactly, for any triangle
+a texel names, in either inner tree, alone and in a batch."""
+import numpy as np
+import pytest
+
+from fornos_b200 import api
+from fornos_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+SPP, LO, HI = 33, 0.001, 0.4
+
+
+def flat(quads, seed):
+    rng = np.random.default_rng(seed)
+    return W.grid_plane(quads, heights=0.1 * rng.uniform(0, 1, (quads + 1) ** 2))
+
+
+# one leaf (no inner tree), one record, remainders, trees of many levels
+@pytest.mark.parametrize("quads,max_tris", [(1, 8), (1, 1), (2, 8), (3, 1), (17, 3), (64, 8), (96, 1)])
+@pytest.mark.parametrize("tree", [api.TREE_SAH, api.TREE_REFERENCE])
+def test_path_start_equals_skip_walk(quads, max_tris, tree):
+    ctx = api.Context(0)
+    mesh = api.Mesh(flat(quads, quads))
+    mesh.compute_vertex_normals()
+    scene = api.Scene.build(ctx, mesh, max_tris)
+    nt, n = 2 * quads * quads, 777
+    rng = np.random.default_rng(5)
+    # every seventh texel misses; the others start on a triangle of their own, some far outside it
+    tidx = (3 * rng.integers(0, nt, n)).astype(np.uint32)
+    tidx[:3] = 0, 3 * (nt - 1), 3 * (nt // 2)
+    tidx[6::7] = api.MISS
+    coords = np.zeros((n, 4), np.float32)
+    coords[:, 1:] = rng.dirichlet((1, 1, 1), n)
+    coords[1::5, 1:] = (3.0, -1.0, -1.0)
+    scene.set_tree(tree)
+    cb, tb = ctx.upload(coords), ctx.upload(tidx)
+    table = ctx.upload(api.samples_cosine(SPP, 16, 3))
+    got = []
+    for traverse in (api.TRAVERSE_ORDERED, api.TRAVERSE_ORDERED | api.EXACT_BOX_TESTS, api.TRAVERSE_SKIP):
+        out, hits = ctx.buffer(4 * n), ctx.buffer(4 * n)
+        api.hemisphere(ctx, scene, cb, tb, api.AO, SPP, LO, HI, table, out, None, hits, None, 0, n, 16, traverse)
+        got.append((out.download(np.uint32, n), hits.download(np.uint32, n)))
+    jobs = [dict(scene=scene, coords=cb, tidx=tb, texel_count=n, spp=SPP, perms=16, min_distance=LO, max_distance=HI,
+                 samples=table, out0=ctx.buffer(4 * n), hits0=ctx.buffer(4 * n)) for _ in range(2)]
+    batch = api.Batch(ctx, jobs, api.AO)
+    batch.run(api.TRAVERSE_ORDERED)
+    got += [(j["out0"].download(np.uint32, n), j["hits0"].download(np.uint32, n)) for j in jobs]
+    ctx.check()
+    assert got[2][1].max() > 0 or nt <= 8
+    for out, hits in got:
+        assert np.array_equal(out, got[2][0]) and np.array_equal(hits, got[2][1])
