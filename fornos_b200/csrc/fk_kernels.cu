@@ -182,6 +182,11 @@ __device__ __forceinline__ void tri_sample(const SceneDev& s, uint32_t t, f3 o, 
   float den = __fsub_rn(__fmul_rn(d00, d11), __fmul_rn(d01, d01));
   const float ny = __fsub_rn(__fmul_rn(d11, d20), __fmul_rn(d01, d21));
   const float nz = __fsub_rn(__fmul_rn(d00, d21), __fmul_rn(d01, d20));
+  // Certain rejections before the divisions (y or z below zero by more than an
+  // underflow, or y + z above 1 by more than the sums' rounding): AO + BN, 500 x
+  // 500 texels, 256 spp, 2.1M triangles 24.8 -> 24.5 ms.
+  const float low = __fmul_rn(den, -1e-30f);
+  if (den > 0.0f && (ny < low || nz < low || __fadd_rn(ny, nz) > __fmul_rn(den, 1.00001f))) return;
   float y = __fdiv_rn(ny, den);
   float z = __fdiv_rn(nz, den);
   float x = __fsub_rn(__fsub_rn(1.0f, y), z);
@@ -684,17 +689,34 @@ __device__ __forceinline__ bool child_maybe(const RayPre& r, const float* ray, f
 }
 
 // Lane state of the ordered traversal in the dynamic schedule.  A lane holds
-// the next inner record to visit (cur) and at most one postponed leaf (pend,
-// a flattened node index); the warp alternates between an inner phase and a
-// leaf phase so that its lanes run the same kind of work together (Aila and
-// Laine's while-while structure with postponed leaves).  Leaves are tested
-// only after their box passed against a threshold no smaller than the
-// current one, and re-checked against the current threshold before their
-// triangles run, so the leaf set is that of the ordered traversal.
+// the next ref of its ray (cur: a record to visit, a leaf that waits, or none)
+// and at most one postponed leaf (pend, a flattened node index); the warp
+// alternates between an inner phase and a leaf phase so that its lanes run the
+// same kind of work together (Aila and Laine's while-while structure with
+// postponed leaves).  Leaves are taken only after their box passed against a
+// threshold no smaller than the current one, and their box is tested exactly
+// against the current threshold before a hit in them counts, so the leaf set
+// is that of the ordered traversal.
 struct OState {
   int32_t cur, pend;
   int sp;
 };
+constexpr int32_t kNoRef = (int32_t)0x80000000;  // no leaf has this ref: a tree has fewer than 2^31 nodes
+
+// Puts a lane's state in order after a visit or a leaf phase: without a next
+// ref it takes the nearest deferred one, and a leaf becomes the postponed one
+// when none is held, so that the lane goes on with the next deferred ref.  A
+// visit then only has to keep the near child and defer the far one; deciding
+// the children's roles (postponed leaf, next record, deferred) in the visit,
+// and leaving a lane that holds a leaf without an inner child idle, took
+// 24.3 against 21.7 ms (AO + BN, 500 x 500 texels, 256 spp, 2.1M triangles).
+__device__ __forceinline__ void next_ref(OState& st, const int32_t* stk) {
+  if (st.cur == kNoRef && st.sp > 0) st.cur = stk[--st.sp];
+  if (st.cur < 0 && st.cur != kNoRef && st.pend < 0) {
+    st.pend = -st.cur - 1;
+    st.cur = st.sp > 0 ? stk[--st.sp] : kNoRef;
+  }
+}
 
 // Deferred entries are record refs, 4 bytes each: the entry distance is not
 // kept.  A popped inner record is visited, which tests its children against
@@ -706,14 +728,11 @@ struct OState {
 // Half the bytes of (ref, distance) pairs keep more of L1 for nodes and
 // triangles, which outweighs the closest-hit search's extra visits.
 
-// Inner phase: tests both children of record `cur` against `thr` and takes
-// them nearer entry first.  Their roles are decided by selects, in the order
-// near child, far child: the first leaf becomes the postponed leaf when none
-// is held, the first inner record the next one to visit, and the rest are
-// deferred by predicated stores (near first, so the far one is popped first),
-// with one overflow check per visit.  Straight-line code keeps the visit free
-// of divergent branches.  TOP: records ref >= top_base are read from the
-// staged copies in shared memory.
+// Inner phase: tests both children of record `cur` against `thr`, keeps the
+// one with the nearer entry as the next ref and defers the other by a
+// predicated store.  Straight-line code keeps the visit free of divergent
+// branches.  TOP: records ref >= top_base are read from the staged copies in
+// shared memory.
 template <bool COUNT, bool FILTER, int S, int STACK = kStack, bool TOP = false>
 __device__ __forceinline__ bool inner_visit(const SceneDev& s, const RayPre& rp, const float* ray, float thr,
                                             OState& st, int32_t* stk,
@@ -731,23 +750,13 @@ __device__ __forceinline__ bool inner_visit(const SceneDev& s, const RayPre& rp,
   const bool h0 = child_maybe<FILTER, S>(rp, ray, mk3(w0.x, w0.z, w2.x), mk3(w0.y, w0.w, w2.y), thr, d0);
   const bool h1 = child_maybe<FILTER, S>(rp, ray, mk3(w1.x, w1.z, w2.z), mk3(w1.y, w1.w, w2.w), thr, d1);
   if (COUNT) tally.box += 2;
-  const bool swap = d1 < d0;
-  const bool hn = swap ? h1 : h0, hf = swap ? h0 : h1;
-  const int32_t rn = __float_as_int(swap ? w3.y : w3.x), rf = __float_as_int(swap ? w3.x : w3.y);
-  const bool nl = hn && rn < 0, ni = hn && rn >= 0, fl = hf && rf < 0, fi = hf && rf >= 0;
-  const bool take_nl = nl && st.pend < 0;
-  const bool take_fl = fl && st.pend < 0 && !take_nl;
-  const bool push_n = nl && !take_nl;
-  const bool push_f = (fl && !take_fl) || (fi && ni);
-  int sp = st.sp;
-  if (push_n && sp < STACK) stk[sp] = rn;
-  sp += push_n;
-  if (push_f && sp < STACK) stk[sp] = rf;
-  sp += push_f;
-  st.pend = take_nl ? -rn - 1 : (take_fl ? -rf - 1 : st.pend);
-  st.cur = ni ? rn : (fi ? rf : -1);
-  st.sp = sp;
-  if (sp > STACK) {
+  const bool both = h0 && h1;
+  const bool swap = h1 && (!h0 || d1 < d0);
+  const int32_t r0 = __float_as_int(w3.x), r1 = __float_as_int(w3.y);
+  if (both && st.sp < STACK) stk[st.sp] = swap ? r0 : r1;
+  st.sp += both;
+  st.cur = h0 || h1 ? (swap ? r1 : r0) : kNoRef;
+  if (st.sp > STACK) {
     atomicOr(status, 1);
     return false;
   }
@@ -817,7 +826,7 @@ __device__ __forceinline__ bool inner_visit4(const SceneDev& s, const RayPre& rp
   st.sp = sp;
   const int32_t rk = keep == 0 ? r0 : (keep == 1 ? r1 : (keep == 2 ? r2 : r3));
   st.pend = keep < 4 ? -rk - 1 : st.pend;
-  st.cur = ni == 0 ? r0 : (ni == 1 ? r1 : (ni == 2 ? r2 : (ni == 3 ? r3 : -1)));
+  st.cur = ni == 0 ? r0 : (ni == 1 ? r1 : (ni == 2 ? r2 : (ni == 3 ? r3 : kNoRef)));
   if (sp > STACK) {
     atomicOr(status, 1);
     return false;
@@ -844,20 +853,28 @@ __device__ __forceinline__ float dist_unkey(uint32_t k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
-// Leaf phase, warp-cooperative.  Every lane holding a postponed leaf tests
-// the leaf's box exactly against its current threshold; the triangles of the
-// leaves that pass are then laid end to end by a warp scan and spread over all
-// 32 lanes: lane j of a round takes item base + j, finds the owning lane by a
-// binary search over the scan and fetches that lane's ray and distance by
-// shuffles.  A hit lowers the owner's distance through a key minimum in
-// shared memory (`skey`, 32 words for this warp).  The closest distance is the
-// minimum over the hits in [lo, best), so neither the order of the tests nor
-// the owner's distance at the start of the phase (which only admits more
-// candidates) changes it.  All lanes of the warp call this; returns whether
-// this lane visited a leaf.  MULTI: lanes may trace different jobs of a
-// batch, whose scenes lie in one concatenated array but whose distance
-// ranges differ, so the owner's minimum distance is read from `wlo` (the
-// warp's lanes' minimum distances in shared memory).
+// Words of shared memory a warp's leaf phase uses: 32 distance keys, then lane
+// and first item of up to 32 owners.
+constexpr int kLeafWords = 96;
+
+// Leaf phase, warp-cooperative.  The triangles of every lane's postponed leaf
+// are laid end to end by a warp scan and spread over all 32 lanes: lane j of a
+// round takes item base + j.  The owners' first items of a round are gathered
+// into one word (an or-reduction), so an item's owner is a population count
+// away and its lane and first triangle are read from shared memory (a binary
+// search over the scan by five dependent shuffles took 2 % more of the kernel).
+// A hit lowers the owner's distance through a key minimum in shared memory.  A
+// leaf's hits count only if the ray hits the leaf's box exactly; that is tested
+// afterwards, in the phases where some leaf has a hit (tested first, for every
+// leaf, it took 1.5 % more: nearly every leaf passes, since the conservative
+// test of the same box came before).  The closest distance is the minimum over
+// the hits in [lo, best), so neither the order of the tests nor the owner's
+// distance at the start of the phase (which only admits more candidates)
+// changes it.  All lanes of the warp call this; returns whether this lane
+// visited a leaf.  MULTI: lanes may trace different jobs of a batch, whose
+// scenes lie in one concatenated array but whose distance ranges differ, so
+// the owner's minimum distance is read from `wlo` (the warp's lanes' minimum
+// distances in shared memory).
 template <bool COUNT, bool FILTER, int S, bool MULTI = false>
 __device__ __forceinline__ bool leaf_phase_warp(const SceneDev& s, const RayPre& rp, const float* wray, float lo,
                                                 float hi, float& best, OState& st, bool active, uint32_t* skey,
@@ -866,17 +883,12 @@ __device__ __forceinline__ bool leaf_phase_warp(const SceneDev& s, const RayPre&
   const int lane = threadIdx.x & 31;
   uint32_t first = 0, cnt = 0;
   const bool mine = active && st.pend >= 0;
-  __syncwarp();  // the lanes' rays, written at their set-up, are read by other lanes below
+  const int32_t leaf = st.pend;
   if (mine) {
-    const float4 L = __ldg(s.node_box + 2 * (size_t)st.pend), H = __ldg(s.node_box + 2 * (size_t)st.pend + 1);
-    float entry;
-    if (COUNT) tally.box++;
-    if (child_hit<FILTER>(rp, ray_o<S>(wray + lane), ray_d<S>(wray + lane), xyz(L), xyz(H), fminf(best, hi),
-                          entry)) {
-      first = as_u32(L.w) / 3;
-      cnt = (as_u32(H.w) - as_u32(L.w)) / 3;
-      if (COUNT) tally.tri += cnt;
-    }
+    const float* b = (const float*)(s.node_box + 2 * (size_t)leaf);
+    first = as_u32(__ldg(b + 3)) / 3;
+    cnt = as_u32(__ldg(b + 7)) / 3 - first;
+    if (COUNT) tally.tri += cnt;
     st.pend = -1;
   }
   uint32_t incl = cnt;
@@ -887,20 +899,26 @@ __device__ __forceinline__ bool leaf_phase_warp(const SceneDev& s, const RayPre&
   const uint32_t total = __shfl_sync(full, incl, 31);
   if (total == 0) return mine;
   skey[lane] = dist_key(best);
-  __syncwarp();
   const uint32_t excl = incl - cnt;
+  const unsigned owners = __ballot_sync(full, cnt > 0);
+  if (cnt > 0) {
+    const uint32_t r = __popc(owners & ((1u << lane) - 1u));
+    skey[32 + r] = lane;
+    skey[64 + r] = first - excl;
+  }
+  __syncwarp();  // these words, and the lanes' rays, written at their set-up, are read by other lanes below
+  uint32_t before = 0;  // owners whose first item lies in an earlier round
   for (uint32_t base = 0; base < total; base += 32) {
     const uint32_t j = base + lane;
-    // owner: the number of lanes whose inclusive count is <= j (steps sum to
-    // 31, so o stays a lane index; for j < total it is the lane holding item j)
-    int o = 0;
-    for (int step = 16; step > 0; step >>= 1) {
-      const uint32_t v = __shfl_sync(full, incl, o + step - 1);
-      if (v <= j) o += step;
-    }
+    // the owner of item j: the last one whose first item is at or before it
+    const uint32_t at = excl - base;
+    const unsigned heads = __reduce_or_sync(full, cnt > 0 && at < 32u ? 1u << at : 0u);
+    const uint32_t r = before + __popc(heads & (0xFFFFFFFFu >> (31 - lane))) - 1;
+    before += __popc(heads);
+    const int o = (int)skey[32 + r];
+    const uint32_t tri = skey[64 + r] + j;
     const f3 ro = ray_o<S>(wray + o), rd = ray_d<S>(wray + o);
     const float ob = __shfl_sync(full, best, o);
-    const uint32_t tri = __shfl_sync(full, first, o) + (j - __shfl_sync(full, excl, o));
     float olo = lo;
     if (MULTI) olo = wlo[o];
     if (j < total) {
@@ -910,18 +928,17 @@ __device__ __forceinline__ bool leaf_phase_warp(const SceneDev& s, const RayPre&
     }
   }
   __syncwarp();
-  if (cnt > 0) best = dist_unkey(skey[lane]);
-  __syncwarp();  // the words are rewritten by the next leaf phase
+  const float t = mine ? dist_unkey(skey[lane]) : best;
+  if (__any_sync(full, t < best)) {  // the warp stays together: without this the rare branch cost 29 %
+    if (t < best) {
+      const float4 L = __ldg(s.node_box + 2 * (size_t)leaf), H = __ldg(s.node_box + 2 * (size_t)leaf + 1);
+      float entry;
+      if (COUNT) tally.box++;
+      if (child_hit<FILTER>(rp, ray_o<S>(wray + lane), ray_d<S>(wray + lane), xyz(L), xyz(H), fminf(best, hi), entry))
+        best = t;
+    }
+  }
   return mine;
-}
-
-// Takes the nearest deferred entry; false when none is left.
-__device__ __forceinline__ bool pop(OState& st, const int32_t* stk) {
-  if (st.sp == 0) return false;
-  const int32_t r = stk[--st.sp];
-  if (r < 0) st.pend = -r - 1;
-  else st.cur = r;
-  return true;
 }
 
 // Start of a ray of the 2-wide ordered traversal at the leaf of the triangle
@@ -956,8 +973,9 @@ __device__ __forceinline__ void path_start(const float4* __restrict__ wide, cons
     path >>= 1;
   }
   st.sp = sp;
-  st.cur = -1;
+  st.cur = kNoRef;
   st.pend = -ref - 1;
+  next_ref(st, stk);
 }
 
 // Skip-pointer walk, one flattened node per call.
@@ -985,11 +1003,9 @@ __device__ __forceinline__ bool skip_step(const SceneDev& s, const RayPre& rp, c
 
 // Inner visits a lane makes per iteration of the trace loop before the warp
 // decides its next phase again (the phase ballots and the refill check are
-// paid once per kInnerVisits visits).
-#ifndef FK_INNER_VISITS
-#define FK_INNER_VISITS 4
-#endif
-constexpr int kInnerVisits = FK_INNER_VISITS;
+// paid once per kInnerVisits visits).  4 / 6 / 8: 21.50 / 21.29 / 21.25 ms (AO +
+// BN, 500 x 500 texels, 256 spp, 2.1M triangles).
+constexpr int kInnerVisits = 8;
 
 // BLOCK: threads per block; STACK: deferred entries per lane (the ordered
 // traversals accept trees of depth below STACK, the 4-wide one of depth up
@@ -1003,8 +1019,8 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 512 ? 2 : 1280 / BLOCK) hemi_t
   const int lane = threadIdx.x & 31;
   const unsigned lower = (1u << lane) - 1u;
   int32_t stk[is_ordered(TRAV) ? STACK : 1];  // deferred record refs
-  __shared__ uint32_t leaf_keys[BLOCK / 32][32];  // leaf-phase distance minimum, per warp
-  uint32_t* skey = leaf_keys[threadIdx.x >> 5];
+  __shared__ uint32_t leaf_words[BLOCK / 32][kLeafWords];
+  uint32_t* skey = leaf_words[threadIdx.x >> 5];
   __shared__ float srays[6 * BLOCK];  // the lanes' ray origins and directions (ray_put)
   __shared__ uint32_t sslot[BLOCK];   // scratch slot of each lane's ray: its texel's row, its sample
   float* const myray = srays + threadIdx.x;
@@ -1020,7 +1036,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 512 ? 2 : 1280 / BLOCK) hemi_t
   RayPre rp = ray_pre(mk3(0.0f, 0.0f, 0.0f), mk3(1.0f, 1.0f, 1.0f));
   float best = FLT_MAX;
   int32_t cur = 0;  // skip walk: node index
-  OState st = {-1, -1, 0};
+  OState st = {kNoRef, -1, 0};
   // counting variant, per warp: iterations, leaf-phase iterations, lanes at
   // work in inner / leaf phases, lanes holding a ray, refills
   unsigned long long wc[6] = {0, 0, 0, 0, 0, 0};
@@ -1066,7 +1082,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 512 ? 2 : 1280 / BLOCK) hemi_t
                   path_start<COUNT, FILTER, BLOCK>(p.s.wide, rp, myray, 0, path, p.hi, st, stk, tally);
                 } else {
                   st.sp = 0;
-                  st.cur = p.s.root_is_leaf ? -1 : (TOP ? (int32_t)top_base : 0);
+                  st.cur = p.s.root_is_leaf ? kNoRef : (TOP ? (int32_t)top_base : 0);
                   st.pend = p.s.root_is_leaf ? 0 : -1;
                 }
                 done = false;
@@ -1094,7 +1110,6 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 512 ? 2 : 1280 / BLOCK) hemi_t
     }
     if (is_ordered(TRAV)) {
       // phase choice, uniform across the warp
-      const bool spec_ok = st.sp < STACK - 4;
       const unsigned need = __ballot_sync(full, active && st.cur >= 0 && st.pend < 0);
       const unsigned leaves = __ballot_sync(full, active && st.pend >= 0);
       const bool leaf_phase = need == 0 || (uint32_t)__popc(leaves) >= p.leaf_batch;
@@ -1108,23 +1123,18 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 512 ? 2 : 1280 / BLOCK) hemi_t
         bool fin = false;
         if (leaf_phase) {
           if (visited) fin = settled<STOP>(best, p.hi);
-        } else if (st.cur >= 0 && (st.pend < 0 || (p.speculate && spec_ok))) {
-          if (!visit_inner<TRAV, COUNT, FILTER, BLOCK, STACK, TOP>(p.s, rp, myray, fminf(best, p.hi), st, stk,
-                                                                    p.status, tally, top_smem, top_base))
-            fin = true;
-          // further visits in the same iteration, continuing from the stack
-          for (int v = 1; v < kInnerVisits && !fin; ++v) {
-            if (st.cur < 0 && st.pend < 0 && !pop(st, stk)) {
+          next_ref(st, stk);
+        } else {
+          for (int v = 0; v < kInnerVisits && st.cur >= 0 && (st.pend < 0 || p.speculate); ++v) {
+            if (!visit_inner<TRAV, COUNT, FILTER, BLOCK, STACK, TOP>(p.s, rp, myray, fminf(best, p.hi), st, stk,
+                                                                      p.status, tally, top_smem, top_base)) {
               fin = true;
               break;
             }
-            if (!(st.cur >= 0 && (st.pend < 0 || (p.speculate && st.sp < STACK - 4)))) break;
-            if (!visit_inner<TRAV, COUNT, FILTER, BLOCK, STACK, TOP>(p.s, rp, myray, fminf(best, p.hi), st, stk,
-                                                                      p.status, tally, top_smem, top_base))
-              fin = true;
+            next_ref(st, stk);
           }
         }
-        if (!fin && st.cur < 0 && st.pend < 0) fin = !pop(st, stk);
+        fin = fin || (st.cur == kNoRef && st.pend < 0);
         if (fin) {
           p.scratch[sslot[threadIdx.x]] = best;
           active = false;
@@ -1468,8 +1478,8 @@ __global__ void __launch_bounds__(256, FK_BATCH_MIN_BLOCKS) batch_trace_kernel(B
   // a launch traces at most the scratch's 2^27 rays: lane indices fit 32 bits
   const uint32_t total = (uint32_t)((p.r1 - p.r0 + p.stride - 1) / p.stride);
   int32_t stk[is_ordered(TRAV) ? kStack : 1];  // deferred record refs
-  __shared__ uint32_t leaf_keys[256 / 32][32];  // leaf-phase distance minimum, per warp
-  uint32_t* skey = leaf_keys[threadIdx.x >> 5];
+  __shared__ uint32_t leaf_words[256 / 32][kLeafWords];
+  uint32_t* skey = leaf_words[threadIdx.x >> 5];
   __shared__ float srays[6 * 256];  // the lanes' ray origins and directions (ray_put)
   float* const myray = srays + threadIdx.x;
   const float* const wray = srays + (threadIdx.x & ~31u);
@@ -1479,7 +1489,7 @@ __global__ void __launch_bounds__(256, FK_BATCH_MIN_BLOCKS) batch_trace_kernel(B
   float best = FLT_MAX, hi = 0.0f;
   int32_t cur = 0;
   uint32_t end = 0;  // skip walk: one past the job's last node
-  OState st = {-1, -1, 0};
+  OState st = {kNoRef, -1, 0};
   const SceneDev& s = p.cat;  // every job's scene, concatenated
   for (;;) {
     unsigned idle = __ballot_sync(full, !active);
@@ -1540,7 +1550,7 @@ __global__ void __launch_bounds__(256, FK_BATCH_MIN_BLOCKS) batch_trace_kernel(B
                   path_start<false, FILTER, 256>(s.wide, rp, myray, J.root2, path, hi, st, stk, tally);
                 } else {
                   st.sp = 0;
-                  st.cur = J.s.root_is_leaf ? -1 : (TRAV == FK_TRAVERSE_ORDERED4 ? J.root4 : J.root2);
+                  st.cur = J.s.root_is_leaf ? kNoRef : (TRAV == FK_TRAVERSE_ORDERED4 ? J.root4 : J.root2);
                   st.pend = J.s.root_is_leaf ? (int32_t)J.node_base : -1;
                 }
                 done = false;
@@ -1564,7 +1574,6 @@ __global__ void __launch_bounds__(256, FK_BATCH_MIN_BLOCKS) batch_trace_kernel(B
     }
     if (exhausted && idle == full) break;
     if (is_ordered(TRAV)) {
-      const bool spec_ok = st.sp < kStack - 4;
       const unsigned need = __ballot_sync(full, active && st.cur >= 0 && st.pend < 0);
       const unsigned leaves = __ballot_sync(full, active && st.pend >= 0);
       const bool leaf_phase = need == 0 || (uint32_t)__popc(leaves) >= p.leaf_batch;
@@ -1575,20 +1584,17 @@ __global__ void __launch_bounds__(256, FK_BATCH_MIN_BLOCKS) batch_trace_kernel(B
         bool fin = false;
         if (leaf_phase) {
           if (visited) fin = settled<STOP>(best, hi);
-        } else if (st.cur >= 0 && (st.pend < 0 || (p.speculate && spec_ok))) {
-          if (!visit_inner<TRAV, false, FILTER, 256>(s, rp, myray, fminf(best, hi), st, stk, p.status, tally))
-            fin = true;
-          for (int v = 1; v < kInnerVisits && !fin; ++v) {  // as in hemi_trace_kernel
-            if (st.cur < 0 && st.pend < 0 && !pop(st, stk)) {
+          next_ref(st, stk);
+        } else {
+          for (int v = 0; v < kInnerVisits && st.cur >= 0 && (st.pend < 0 || p.speculate); ++v) {
+            if (!visit_inner<TRAV, false, FILTER, 256>(s, rp, myray, fminf(best, hi), st, stk, p.status, tally)) {
               fin = true;
               break;
             }
-            if (!(st.cur >= 0 && (st.pend < 0 || (p.speculate && st.sp < kStack - 4)))) break;
-            if (!visit_inner<TRAV, false, FILTER, 256>(s, rp, myray, fminf(best, hi), st, stk, p.status, tally))
-              fin = true;
+            next_ref(st, stk);
           }
         }
-        if (!fin && st.cur < 0 && st.pend < 0) fin = !pop(st, stk);
+        fin = fin || (st.cur == kNoRef && st.pend < 0);
         if (fin) {
           p.scratch[sslot[threadIdx.x]] = best;
           active = false;
