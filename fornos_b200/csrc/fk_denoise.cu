@@ -64,6 +64,12 @@ __device__ __forceinline__ float gelu(float z, float& dz) {
   return (0.5f * z) * (1.0f + th);
 }
 
+// The same value without the derivative.
+__device__ __forceinline__ float gelu_value(float z) {
+  const float u = 0.7978845608028654f * (z + 0.044715f * ((z * z) * z));
+  return (0.5f * z) * (1.0f + tanhf(u));
+}
+
 // Octahedral encoding of a direction (zero or non-finite vectors map to 0).
 __device__ __forceinline__ float2 oct_encode(float x, float y, float z) {
   const float s = (fabsf(x) + fabsf(y)) + fabsf(z);
@@ -80,30 +86,47 @@ __device__ __forceinline__ float2 oct_encode(float x, float y, float z) {
 
 __device__ __forceinline__ float clamp4(float v) { return fminf(fmaxf(v, -4.0f), 4.0f); }
 
+// A texel's own terms of its neighbours' features: pixel coordinates,
+// position and spacing.
+struct Centre {
+  int x, y;
+  float px, py, pz, spacing;
+};
+__device__ __forceinline__ Centre centre_of(const float4* __restrict__ f1, const float4* __restrict__ f2, uint32_t w,
+                                            uint32_t p) {
+  Centre c = {0, 0, 0.0f, 0.0f, 0.0f, 0.0f};
+  if (p == kNoTexel) return c;
+  const float4 b = __ldg(f1 + p);
+  c.y = (int)(p / w);
+  c.x = (int)(p - (uint32_t)c.y * w);
+  c.px = b.x;
+  c.py = b.y;
+  c.pz = b.z;
+  c.spacing = __ldg(f2 + p).z;
+  return c;
+}
+
 // The 10 features of neighbour j (< 25, row-major over the 5 x 5 window) of
-// the texel at pixel p; zeros outside the texture, without a mapping hit, or
-// for p = kNoTexel.
+// the texel at pixel p with centre terms c; zeros outside the texture, without
+// a mapping hit, or for p = kNoTexel.
 __device__ __forceinline__ void neighbour_features(const float4* __restrict__ f0, const float4* __restrict__ f1,
                                                    const float4* __restrict__ f2, uint32_t w, uint32_t h, uint32_t p,
-                                                   int j, float (&v)[10]) {
+                                                   const Centre& c, int j, float (&v)[10]) {
 #pragma unroll
   for (int k = 0; k < 10; ++k) v[k] = 0.0f;
   if (p == kNoTexel) return;
-  const int cx = (int)(p % w), cy = (int)(p / w);
-  const int x = cx + j % 5 - 2, y = cy + j / 5 - 2;
+  const int jy = j / 5, x = c.x + (j - 5 * jy) - 2, y = c.y + jy - 2;
   if (x < 0 || y < 0 || x >= (int)w || y >= (int)h) return;
   const uint32_t q = (uint32_t)y * w + (uint32_t)x;
-  const float4 a = __ldg(f0 + q);
+  const float4 a = __ldg(f0 + q), b = __ldg(f1 + q), n = __ldg(f2 + q);
   if (!(a.w > 0.0f)) return;
-  const float4 c = __ldg(f1 + p), b = __ldg(f1 + q), n = __ldg(f2 + q);
-  const float sp = __ldg(f2 + p).z;  // centre texel spacing
   v[0] = a.x;
   v[1] = a.y;
   v[2] = a.z;
-  if (sp > 0.0f) {
-    v[3] = clamp4((b.x - c.x) / sp);
-    v[4] = clamp4((b.y - c.y) / sp);
-    v[5] = clamp4((b.z - c.z) / sp);
+  if (c.spacing > 0.0f) {
+    v[3] = clamp4((b.x - c.px) / c.spacing);
+    v[4] = clamp4((b.y - c.py) / c.spacing);
+    v[5] = clamp4((b.z - c.pz) / c.spacing);
   }
   v[6] = n.x;
   v[7] = n.y;
@@ -118,7 +141,7 @@ __device__ __forceinline__ void assemble_row(const float4* __restrict__ f0, cons
                                              int lane, uint32_t* dst) {
   if (lane < 25) {
     float v[10];
-    neighbour_features(f0, f1, f2, w, h, p, lane, v);
+    neighbour_features(f0, f1, f2, w, h, p, centre_of(f1, f2, w, p), lane, v);
 #pragma unroll
     for (int k = 0; k < 5; ++k) dst[5 * lane + k] = pack2(v[2 * k], v[2 * k + 1]);
   } else if (lane == 25) {
@@ -704,21 +727,35 @@ __global__ void __launch_bounds__(256, 2) dn_apply_kernel(ApplyArgs a) {
 // tcgen05.commit arrives on; every wait on it is bounded and a timeout stops
 // the kernel with status bit 16 after freeing its tensor memory.
 namespace tc {
-// 16 warps: all gather input rows; for the epilogues, warps w, w + 4, w + 8 and
-// w + 12 share TMEM lane quarter w % 4 (the only lanes a warp may read) and
-// split its 64 accumulator columns 16 each.
+// 16 warps: all assemble input rows; for the epilogues, warps w, w + 4, w + 8
+// and w + 12 share TMEM lane quarter w % 4 (the only lanes a warp may read) and
+// split its 64 accumulator columns 16 each.  106 KB of shared memory and 64
+// registers a thread let two CTAs share an SM, so that one's assembly and
+// epilogues run while the other waits for its tensor-core work; for that the
+// hidden layers' operands lie in the input rows' space, which is free once
+// layer 1 is done.
 constexpr uint32_t kThreads = 512;
+constexpr uint32_t kCtasPerSm = 2;
 constexpr uint32_t kTmemCols = 128;  // layer 1 / 3 accumulators at column 0, layer 2 at column 64
 constexpr uint32_t kA1 = 0;                  // 128 x 256 bf16
-constexpr uint32_t kW1 = kA1 + 128 * 256 * 2;  // 64 x 256
-constexpr uint32_t kA2 = kW1 + 64 * 256 * 2;   // 128 x 64
+constexpr uint32_t kA2 = kA1;                  // 128 x 64
 constexpr uint32_t kA3 = kA2 + 128 * 64 * 2;   // 128 x 64
-constexpr uint32_t kW2 = kA3 + 128 * 64 * 2;   // 64 x 64
+constexpr uint32_t kW1 = kA1 + 128 * 256 * 2;  // 64 x 256
+constexpr uint32_t kW2 = kW1 + 64 * 256 * 2;   // 64 x 64
 constexpr uint32_t kW3 = kW2 + 64 * 64 * 2;    // 16 x 64, rows 4..15 zero
 constexpr uint32_t kBar = kW3 + 16 * 64 * 2;   // mbarrier (8 bytes)
 constexpr uint32_t kSlot = kBar + 8;           // allocated TMEM address
 constexpr uint32_t kBytes = kSlot + 8;
 constexpr uint32_t kWaitLimit = 1u << 22;
+
+// Order of the inputs along K for rows assembled from the feature image: the
+// first eight features of neighbour j in columns 8 j .. 8 j + 7 (one 16-byte
+// store), its last two in 200 + 2 j, 201 + 2 j; 250 .. 255 are the pad.  The
+// input column (10 j + feature) at place k:
+__device__ __forceinline__ uint32_t input_column(uint32_t k) {
+  if (k < 200) return 10 * (k >> 3) + (k & 7);
+  return k < 250 ? 10 * ((k - 200) >> 1) + 8 + (k & 1) : k;
+}
 
 // Byte offset of element (r, k) in a K-major core-matrix tile whose rows hold
 // `kdim` elements: core matrices of 8 rows x 8 elements, 128 bytes each,
@@ -799,10 +836,9 @@ __device__ __forceinline__ void hidden_epilogue(uint32_t taddr, uint32_t c0, con
     uint32_t w4[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      float dz;
       const uint32_t c = c0 + 8 * h + 2 * e;
-      const float a0 = gelu(v[8 * h + 2 * e] + __ldg(bias + c), dz);
-      const float a1 = gelu(v[8 * h + 2 * e + 1] + __ldg(bias + c + 1), dz);
+      const float a0 = gelu_value(v[8 * h + 2 * e] + __ldg(bias + c));
+      const float a1 = gelu_value(v[8 * h + 2 * e + 1] + __ldg(bias + c + 1));
       w4[e] = pack2(a0, a1);
     }
     *(uint4*)(dst + core_off(row, c0 + 8 * h, 64)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
@@ -810,7 +846,14 @@ __device__ __forceinline__ void hidden_epilogue(uint32_t taddr, uint32_t c0, con
 }
 }  // namespace tc
 
-__global__ void __launch_bounds__(tc::kThreads, 1) dn_apply_tc_kernel(ApplyArgs a, int* status) {
+// Bound by the assembly of the input rows and the GELUs of the epilogues, the
+// matrix work is a few percent.  Assembly: a thread owns one row (lanes hold
+// consecutive texels, so a neighbour's features are consecutive in memory and
+// the 16-byte operand stores hit all banks) and every fourth neighbour.  One
+// warp per row with a lane per neighbour, scattered loads and 4-byte stores and
+// one CTA per SM took 593 us for a 1024 x 1024 map (750k texels); this takes
+// 288 us (issue 57 % active, 7.4k thread instructions a texel, tanhf most of them).
+__global__ void __launch_bounds__(tc::kThreads, tc::kCtasPerSm) dn_apply_tc_kernel(ApplyArgs a, int* status) {
   extern __shared__ __align__(128) unsigned char sm[];
   const uint32_t sb = (uint32_t)__cvta_generic_to_shared(sm);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -818,9 +861,17 @@ __global__ void __launch_bounds__(tc::kThreads, 1) dn_apply_tc_kernel(ApplyArgs 
   const uint32_t cols = 16 * (warp >> 2);     // this warp's accumulator columns in an epilogue
   const uint32_t row = 32 * quarter + lane;   // tile row = TMEM lane of this thread
   // weights into the core-matrix layout (16-byte chunks of 8 elements)
-  for (uint32_t i = threadIdx.x; i < 64 * 32; i += tc::kThreads) {
-    const uint32_t n = i / 32, kg = i % 32;
-    *(uint4*)(sm + tc::kW1 + tc::core_off(n, 8 * kg, 256)) = __ldg((const uint4*)a.wt.w1 + n * 32 + kg);
+  if (a.rows) {
+    for (uint32_t i = threadIdx.x; i < 64 * 32; i += tc::kThreads) {
+      const uint32_t n = i / 32, kg = i % 32;
+      *(uint4*)(sm + tc::kW1 + tc::core_off(n, 8 * kg, 256)) = __ldg((const uint4*)a.wt.w1 + n * 32 + kg);
+    }
+  } else {
+    for (uint32_t i = threadIdx.x; i < 64 * 256; i += tc::kThreads) {
+      const uint32_t n = i / 256, k = i % 256;
+      *(uint16_t*)(sm + tc::kW1 + tc::core_off(n, k, 256)) =
+          __ldg((const uint16_t*)a.wt.w1 + n * 256 + tc::input_column(k));
+    }
   }
   for (uint32_t i = threadIdx.x; i < 64 * 8; i += tc::kThreads) {
     const uint32_t n = i / 8, kg = i % 8;
@@ -856,26 +907,29 @@ __global__ void __launch_bounds__(tc::kThreads, 1) dn_apply_tc_kernel(ApplyArgs 
   bool failed = false;  // a bounded wait ran out (agreed by all threads)
   for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const uint32_t first = a.offset + tile * dn::kRows;
-    // input rows: warp w assembles rows 8w .. 8w + 7
-    for (int rr = 0; rr < 8; ++rr) {
-      const uint32_t r = (uint32_t)(warp * 8 + rr), i = first + r;
-      if (a.rows) {
+    if (a.rows) {
+      // given rows: warp w copies rows 8w .. 8w + 7
+      for (int rr = 0; rr < 8; ++rr) {
+        const uint32_t r = (uint32_t)(warp * 8 + rr), i = first + r;
         const uint4 v = i < end ? __ldg((const uint4*)(a.rows + (size_t)i * (dn::kK1 / 2)) + lane)
                                 : make_uint4(0, 0, 0, 0);
         *(uint4*)(sm + tc::kA1 + tc::core_off(r, 8 * lane, 256)) = v;
-      } else {
-        uint32_t px = i < end ? __ldg(a.indices + i) : kNoTexel;
-        if (px >= a.w * a.h) px = kNoTexel;
-        if (lane < 25) {
-          float v[10];
-          neighbour_features(a.f0, a.f1, a.f2, a.w, a.h, px, lane, v);
-#pragma unroll
-          for (int k = 0; k < 5; ++k)
-            *(uint32_t*)(sm + tc::kA1 + tc::core_off(r, 10 * lane + 2 * k, 256)) = pack2(v[2 * k], v[2 * k + 1]);
-        } else if (lane == 25) {
-          for (int k = 250; k < 256; k += 2) *(uint32_t*)(sm + tc::kA1 + tc::core_off(r, k, 256)) = 0u;
-        }
       }
+    } else {
+      const uint32_t r = threadIdx.x & 127, part = threadIdx.x >> 7, i = first + r;
+      uint32_t px = i < end ? __ldg(a.indices + i) : kNoTexel;
+      if (px >= a.w * a.h) px = kNoTexel;
+      const Centre c = centre_of(a.f1, a.f2, a.w, px);
+#pragma unroll 2
+      for (uint32_t j = part; j < 25; j += 4) {
+        float v[10];
+        neighbour_features(a.f0, a.f1, a.f2, a.w, a.h, px, c, (int)j, v);
+        *(uint4*)(sm + tc::kA1 + tc::core_off(r, 8 * j, 256)) =
+            make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+        *(uint32_t*)(sm + tc::kA1 + tc::core_off(r, 200 + 2 * j, 256)) = pack2(v[8], v[9]);
+      }
+      if (part == 3)
+        for (uint32_t k = 250; k < 256; k += 2) *(uint32_t*)(sm + tc::kA1 + tc::core_off(r, k, 256)) = 0u;
     }
     tc::fence_proxy();
     tc::sync_all();
@@ -1172,7 +1226,7 @@ cudaError_t launch_apply_tc(cudaStream_t st, int sm_count, const float4* image, 
   a.y_out = y_out;
   a.rows = rows;
   const uint32_t tiles = (count + kRows - 1) / kRows;
-  const uint32_t blocks = std::min<uint32_t>(tiles, (uint32_t)sm_count);  // one CTA per SM (141 KB of shared memory)
+  const uint32_t blocks = std::min<uint32_t>(tiles, (uint32_t)sm_count * tc::kCtasPerSm);
   dn_apply_tc_kernel<<<blocks, tc::kThreads, tc::kBytes, st>>>(a, status);
   return cudaGetLastError();
 }
