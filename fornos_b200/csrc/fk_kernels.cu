@@ -42,6 +42,9 @@ static SceneDev dev_of(const fk_scene* s) {
   d.wide4 = s->wide4;
   d.rec = s->tri_rec;
   d.rec_bary = s->tri_rec + s->corner_count / 3;
+  d.map_pad = s->map_pad;
+  d.chain_box = s->chain_box;
+  d.sah = s->tree_wide[FK_TREE_SAH];
   d.tri_path = s->tri_path;
   d.node_count = s->node_count;
   d.root_is_leaf = s->root_is_leaf;
@@ -1983,9 +1986,217 @@ __device__ float walk_twoside(const SceneDev& s, f3 o, f3 d, float mint, uint32_
   return mint;
 }
 
-// max_d: the walks' initial closest distance (FLT_MAX in the shaders); a
-// miss writes t = FLT_MAX whatever it is.
+// Mapping over the scene's inner tree in place of the two skip-pointer walks,
+// with their result bit for bit.  Both walks of a texel meet the same hits
+// with t and -t (dot(-d, n) = -dot(d, n), and the hit point is the same), so one
+// traversal of the whole line serves both, nearest boxes first.
+//
+// What the walks return: a walk visits the leaves in order, those whose box
+// and whose ancestors' boxes it enters at a distance below its closest hit so
+// far, which is never below the smallest hit distance t* of all triangles.  If
+// every leaf with a hit at t* is entered that way at a <= t*, the first of them
+// is visited (it is met with the closest hit still above t*), its first
+// triangle at t* is taken and nothing replaces it: the result is the smallest
+// (t, walk, corner).  The traversal finds that triple and checks a <= t* with
+// the walks' own box test on the box that the leaf and its ancestors have in
+// common (chain_box; the flattened boxes are rounded from centre and half size
+// and do not nest exactly; the test is monotone, so each of them is entered no
+// later).  A texel for which it fails (a hit that rounds to before its leaf's
+// box, a ray in a box face) takes the walks.
+//
+// It finds every hit up to t*: a hit lies within map_pad + 128 u M' of its
+// triangle's box (u = 2^-24, M' the largest coordinate of scene and origin).
+// With L = |v0| + |v1| and s = sin^2 of the edges' angle, the binary64
+// barycentrics put the hit point's projection within 1e-5 (|x|, |y| and |z|
+// slack, 2.1e-5 L) of the triangle, and the point is off the triangle's plane
+// by at most 39 u M' + 7.1 u |p - a| (rounding of t and p, see below) plus
+// |p - a| 16 u / sqrt(s) for the rounded normal, 10.4 u M' more to the ray
+// itself: map_pad = max L (2.1e-5 + 17 u / sqrt(s)); a triangle may stick out of
+// its rounded leaf box by 8 u M', and 128 u leaves 67 u M' for the slab values.  (an and pn: 3.1 u each of a Euclidean norm of at most
+// sqrt(3) M', their difference u, nd 3.1 u of t, p 2 u (t + |p|).)  A slab value is one fused
+// multiply-add on face and offset, off by at most 5.1 u M' |1 / d|; an axis with
+// |d| < 2^-100 has 1 / d replaced by 2^100 (t < 2^27, so the ray moves less than
+// 2^-73 along it, and the padded faces are as good as infinitely far or behind).
+// map_pad_kernel gives an infinite bound where this does not hold: s below
+// 2^-24, edges outside [2^-25, 2^25], a triangle outside its leaf's box or the
+// root's coordinates (an uploaded scene); a triangle whose normal is NaN is
+// never hit.  Directions far from unit length and
+// coordinates from 2^24 up take the walks too.
+//
+// Bound by the latency of the record and triangle loads.  The walks divide six
+// times a node and visit hundreds of the reference tree's nodes a ray.
+// 2048 x 2048 texels on the 2.1M-triangle heightfield: 4.71 -> 1.03 ms; 128 x 128 texels
+// on a 9k-triangle sphere: 283 -> 59 us.
+__global__ void map_pad_kernel(const float4* __restrict__ lo, const float4* __restrict__ hi,
+                               const uint32_t* __restrict__ jump, const float4* __restrict__ pos4,
+                               const float4* __restrict__ rec, uint32_t nodes, uint32_t* __restrict__ pad,
+                               float4* __restrict__ chain) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  float p = 0.0f;
+  if (i < nodes) {
+    const float4 L = lo[i], H = hi[i], RL = lo[0], RH = hi[0];
+    const float M = fmaxf(fmaxf(fmaxf(fabsf(RL.x), fabsf(RH.x)), fmaxf(fabsf(RL.y), fabsf(RH.y))),
+                          fmaxf(fabsf(RL.z), fabsf(RH.z)));
+    const float inf = __int_as_float(0x7f800000), tol = __fmul_rn(M, 4.76837158e-07f);  // 8 u
+    auto within = [&](f3 a, f3 b) {
+      return a.x >= L.x - tol && a.y >= L.y - tol && a.z >= L.z - tol && b.x <= H.x + tol && b.y <= H.y + tol &&
+             b.z <= H.z + tol;
+    };
+    if (as_u32(L.w) < as_u32(H.w)) {  // a leaf: down to it from the root
+      f3 cl = xyz(L), ch = xyz(H);
+      for (uint32_t c = 0; c < i;) {
+        if (jump[c] <= i) {
+          c = jump[c];
+        } else {
+          cl = vmax(cl, xyz(lo[c]));
+          ch = vmin(ch, xyz(hi[c]));
+          ++c;
+        }
+      }
+      chain[2 * (size_t)i] = make_float4(cl.x, cl.y, cl.z, 0.0f);
+      chain[2 * (size_t)i + 1] = make_float4(ch.x, ch.y, ch.z, 0.0f);
+    }
+    for (uint32_t k = as_u32(L.w); k < as_u32(H.w); k += 3) {
+      const f3 a = xyz(pos4[k]), b = xyz(pos4[k + 1]), c = xyz(pos4[k + 2]);
+      if (!within(vmin(vmin(a, b), c), vmax(vmax(a, b), c))) p = inf;
+      const float4 n = rec[k / 3];
+      if (n.x != n.x || n.y != n.y || n.z != n.z) continue;
+      const double v0x = (double)b.x - a.x, v0y = (double)b.y - a.y, v0z = (double)b.z - a.z;
+      const double v1x = (double)c.x - a.x, v1y = (double)c.y - a.y, v1z = (double)c.z - a.z;
+      const double d00 = v0x * v0x + v0y * v0y + v0z * v0z, d11 = v1x * v1x + v1y * v1y + v1z * v1z;
+      const double x = v0y * v1z - v0z * v1y, y = v0z * v1x - v0x * v1z, z = v0x * v1y - v0y * v1x;
+      const double s = (x * x + y * y + z * z) / (d00 * d11);
+      const double edge2 = 8.8817841970012523e-16;  // 2^-50
+      const bool ok = s >= 5.9604644775390625e-08 && d00 >= edge2 && d11 >= edge2 && d00 <= 1.0 / edge2 &&
+                      d11 <= 1.0 / edge2 && fabsf(a.x) <= M && fabsf(a.y) <= M && fabsf(a.z) <= M;
+      const double q = (sqrt(d00) + sqrt(d11)) * (2.1e-5 + 17.0 * 5.9604644775390625e-08 / sqrt(s));
+      p = fmaxf(p, ok && q <= 0.05 * M ? __double2float_ru(q) : inf);
+    }
+  }
+  for (int d = 16; d > 0; d >>= 1) p = fmaxf(p, __shfl_xor_sync(0xFFFFFFFFu, p, d));
+  if ((threadIdx.x & 31) == 0 && p > 0.0f) atomicMax(pad, __float_as_uint(p));
+}
+
+int launch_map_pad(fk_ctx* ctx, fk_scene* s) {
+  const cudaError_t e = cudaMemsetAsync(s->map_pad, 0, sizeof(float), ctx->stream);
+  if (e != cudaSuccess) return fk_cuda_fail(ctx, e, "mapping bound");
+  map_pad_kernel<<<(s->node_count + 255) / 256, 256, 0, ctx->stream>>>(s->node_lo, s->node_hi, s->node_jump, s->pos4,
+                                                                       s->tri_rec, s->node_count, (uint32_t*)s->map_pad, s->chain_box);
+  return fk_after_launch(ctx, "map_pad_kernel");
+}
+
+// One axis of the padded slab test: value of a face f is fma(f, inv, -ol) for
+// the lower face and fma(f, inv, -oh) for the upper one.
+__device__ __forceinline__ void line_axis(float o, float d, float pad, float& inv, float& ol, float& oh) {
+  inv = fabsf(d) >= 7.8886091e-31f ? __frcp_rn(d) : 1.26765060e30f;  // 2^-100, 2^100
+  const float oi = __fmul_rn(o, inv), m = __fmul_rn(pad, inv);
+  ol = __fadd_rn(oi, m);
+  oh = __fsub_rn(oi, m);
+}
+
+// The smallest (|t|, walk, corner) hit below max_d over the whole line, or
+// false when the texel needs the walks.  On a miss id stays kMiss.
 template <int CULL>
+__device__ bool map_line(const SceneDev& s, f3 o, f3 d, float max_d, float& t, uint32_t& id, f3& w) {
+  const float4 RL = __ldg(s.node_lo), RH = __ldg(s.node_hi);
+  const float root = fmaxf(fmaxf(fmaxf(fabsf(RL.x), fabsf(RH.x)), fmaxf(fabsf(RL.y), fabsf(RH.y))),
+                           fmaxf(fabsf(RL.z), fabsf(RH.z)));
+  const float far = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fabsf(o.z));
+  const float len = fmaxf(fmaxf(fabsf(d.x), fabsf(d.y)), fabsf(d.z));
+  const float M = fmaxf(root, far), bound = __ldg(s.map_pad);
+  // sums so that a NaN in any component fails (fmaxf drops it)
+  const bool finite = fabsf(o.x) + fabsf(o.y) + fabsf(o.z) < 5.0e7f && fabsf(d.x) + fabsf(d.y) + fabsf(d.z) < 4.0f;
+  if (!(finite && M < 16777216.0f && len >= 0.5f && bound <= 0.05f * root)) return false;
+  const float pad = __fadd_rn(bound, __fmul_rn(M, 7.62939453e-06f));  // 128 u
+  f3 inv, ol, oh;
+  line_axis(o.x, d.x, pad, inv.x, ol.x, oh.x);
+  line_axis(o.y, d.y, pad, inv.y, ol.y, oh.y);
+  line_axis(o.z, d.z, pad, inv.z, ol.z, oh.z);
+  // distance (from the origin, either way) at which the line can be in the box; negative: never
+  auto reach = [&](f3 lo, f3 hi) {
+    // both offsets of a face: with inv < 0 the lower face is the far one
+    const float t1x = __fmaf_rn(lo.x, inv.x, -ol.x), t2x = __fmaf_rn(hi.x, inv.x, -oh.x);
+    const float t1y = __fmaf_rn(lo.y, inv.y, -ol.y), t2y = __fmaf_rn(hi.y, inv.y, -oh.y);
+    const float t1z = __fmaf_rn(lo.z, inv.z, -ol.z), t2z = __fmaf_rn(hi.z, inv.z, -oh.z);
+    const float a = fmaxf(fmaxf(fminf(t1x, t2x), fminf(t1y, t2y)), fminf(t1z, t2z));
+    const float b = fminf(fminf(fmaxf(t1x, t2x), fmaxf(t1y, t2y)), fmaxf(t1z, t2z));
+    return a <= b ? fmaxf(fmaxf(a, -b), 0.0f) : -1.0f;
+  };
+  int32_t stk_ref[kMaxOrderedDepth + 1];
+  float stk_dist[kMaxOrderedDepth + 1];
+  int sp = 0;
+  float best = max_d;
+  uint32_t corner = kMiss;
+  int walk = 0;  // 0: along d, 1: along -d
+  bool sure = true;
+  int32_t cur = 0;
+  for (;;) {
+    while (cur >= 0) {
+      const float4* r = s.sah + 4 * (size_t)cur;
+      const float4 w0 = __ldg(r), w1 = __ldg(r + 1), w2 = __ldg(r + 2), w3 = __ldg(r + 3);
+      const float d0 = reach(mk3(w0.x, w0.z, w2.x), mk3(w0.y, w0.w, w2.y));
+      const float d1 = reach(mk3(w1.x, w1.z, w2.z), mk3(w1.y, w1.w, w2.w));
+      const bool h0 = d0 >= 0.0f && d0 <= best, h1 = d1 >= 0.0f && d1 <= best;
+      const int32_t r0 = __float_as_int(w3.x), r1 = __float_as_int(w3.y);
+      const bool swap = h1 && (!h0 || d1 < d0);
+      if (h0 && h1) {  // at most one entry a level
+        stk_ref[sp] = swap ? r0 : r1;
+        stk_dist[sp] = swap ? d0 : d1;
+        ++sp;
+      }
+      cur = swap ? r1 : r0;
+      if (!h0 && !h1) {
+        cur = kNoRef;
+        while (sp > 0) {
+          --sp;
+          if (stk_dist[sp] <= best) {
+            cur = stk_ref[sp];
+            break;
+          }
+        }
+      }
+    }
+    if (cur == kNoRef) break;
+    {
+      const float* range = (const float*)(s.node_box + 2 * (size_t)(-(cur + 1)));
+      for (uint32_t k = as_u32(__ldg(range + 3)), e = as_u32(__ldg(range + 7)); k < e; k += 3) {
+        const float4 A = __ldg(s.rec + k / 3);
+        const f3 n = xyz(A);
+        const float nd = dot(d, n);
+        if (CULL ? !(nd > 0.0f) : !(fabsf(nd) > 0.0f)) continue;
+        const float th = __fdiv_rn(__fsub_rn(A.w, dot(o, n)), nd);
+        const float at = fabsf(th);
+        const int wk = th >= 0.0f ? 0 : 1;
+        if (!(at < best || (at == best && corner != kMiss && (wk < walk || (wk == walk && k < corner))))) continue;
+        const f3 q = bary_f64(add(o, scale(d, th)), xyz(__ldg(s.pos4 + k)), xyz(__ldg(s.pos4 + k + 1)),
+                              xyz(__ldg(s.pos4 + k + 2)));
+        if (!bary_ok_map(q)) continue;
+        const float4 cl = __ldg(s.chain_box + 2 * (size_t)(-(cur + 1))), ch = __ldg(s.chain_box + 2 * (size_t)(-(cur + 1)) + 1);
+        const bool visited = ray_box(o, wk ? neg(d) : d, xyz(cl), xyz(ch)) <= at;
+        sure = at < best ? visited : sure && visited;
+        best = at;
+        corner = k;
+        walk = wk;
+        w = q;
+      }
+    }
+    cur = kNoRef;
+    while (sp > 0) {
+      --sp;
+      if (stk_dist[sp] <= best) {
+        cur = stk_ref[sp];
+        break;
+      }
+    }
+  }
+  t = best;
+  id = corner;
+  return sure;
+}
+
+// max_d: the walks' initial closest distance (FLT_MAX in the shaders); a
+// miss writes t = FLT_MAX whatever it is.  TREE: map_line first.
+template <int CULL, bool TREE>
 __global__ void __launch_bounds__(128) meshmap_kernel(SceneDev s, const float4* __restrict__ pix, float max_d,
                                                       uint32_t offset, uint32_t count, float4* __restrict__ coords,
                                                       uint32_t* __restrict__ tidx) {
@@ -1996,12 +2207,17 @@ __global__ void __launch_bounds__(128) meshmap_kernel(SceneDev s, const float4* 
   uint32_t id = kMiss;
   f3 w = mk3(0.0f, 0.0f, 0.0f);
   float t = max_d;
-  if (CULL) {
-    walk_oneside<+1>(s, p, d, t, id, w);
-    walk_oneside<-1>(s, p, neg(d), t, id, w);
-  } else {
-    t = fminf(t, walk_twoside(s, p, d, t, id, w));
-    t = fminf(t, walk_twoside(s, p, neg(d), t, id, w));
+  if (!TREE || !map_line<CULL>(s, p, d, max_d, t, id, w)) {
+    id = kMiss;
+    w = mk3(0.0f, 0.0f, 0.0f);
+    t = max_d;
+    if (CULL) {
+      walk_oneside<+1>(s, p, d, t, id, w);
+      walk_oneside<-1>(s, p, neg(d), t, id, w);
+    } else {
+      t = fminf(t, walk_twoside(s, p, d, t, id, w));
+      t = fminf(t, walk_twoside(s, p, neg(d), t, id, w));
+    }
   }
   if (id == kMiss) t = FLT_MAX;
   coords[g] = make_float4(t, w.x, w.y, w.z);
@@ -2012,8 +2228,11 @@ int launch_meshmap(fk_ctx* ctx, const fk_scene* s, const fk_texel_map* m, int cu
                    uint32_t count, float4* coords, uint32_t* tidx) {
   if (count == 0) return FK_OK;
   uint32_t blocks = (count + 127) / 128;
-  if (cull) meshmap_kernel<1><<<blocks, 128, 0, ctx->stream>>>(dev_of(s), m->pix, max_d, offset, count, coords, tidx);
-  else meshmap_kernel<0><<<blocks, 128, 0, ctx->stream>>>(dev_of(s), m->pix, max_d, offset, count, coords, tidx);
+  // a rebuilt tree (kept only where it fits the stack; a single leaf has none) and coordinates below 2^24
+  const bool tree = s->tree_wide[FK_TREE_SAH] && !s->root_is_leaf && s->filter_ok;
+  auto kern = cull ? (tree ? meshmap_kernel<1, true> : meshmap_kernel<1, false>)
+                   : (tree ? meshmap_kernel<0, true> : meshmap_kernel<0, false>);
+  kern<<<blocks, 128, 0, ctx->stream>>>(dev_of(s), m->pix, max_d, offset, count, coords, tidx);
   return fk_after_launch(ctx, "meshmap_kernel");
 }
 

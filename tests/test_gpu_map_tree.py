@@ -1,0 +1,89 @@
+"""Mesh mapping over the inner tree against the skip-pointer walks, bit for
+bit.  A direction eight times as long takes the walks (the tree route asks for
+about unit length) and every operation on it is the same but for an exact power
+of two, so both routes run on the same rays and distances differ by that
+factor alone."""
+import numpy as np
+import pytest
+
+from fornos_b200 import api
+from fornos_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def soup(n, seed, size):
+    """Triangles of all shapes: ordinary ones, slivers, repeated corners,
+    collinear corners, identical triangles, one as large as the scene."""
+    rng = np.random.default_rng(seed)
+    c = rng.uniform(-1, 1, (n, 1, 3))
+    p = (c + size * rng.normal(size=(n, 3, 3))).astype(np.float32)
+    p[1::7, 2] = p[1::7, 1] + (p[1::7, 0] - p[1::7, 1]) * np.float32(1e-3) + np.float32(1e-6)
+    p[2::7, 2] = p[2::7, 1]
+    p[3::7, 2] = 0.5 * (p[3::7, 0] + p[3::7, 1])
+    p[4::14] = p[4]
+    p[-1] = [[-1, -1, 0], [1, -1, 0], [0, 1, 0]]
+    tri = np.arange(3 * n).reshape(-1, 3)
+    return W.MeshArrays(p.reshape(-1, 3), np.zeros((1, 2)), np.tile([[0, 0, 1]], (3 * n, 1)),
+                        np.stack([np.arange(3 * n), np.zeros(3 * n), np.arange(3 * n)], -1), tri)
+
+
+MESHES = {
+    "sphere": lambda: W.sphere_pair(seed=3, hi_seg=(256, 96))[1],     # thin triangles round the poles
+    "heights": lambda: W.plane_pair(seed=4, hi_quads=64, bumps=20)[1],
+    "flat": lambda: W.grid_plane(32),                                 # every hit lies in its leaf's box face
+    "soup": lambda: soup(4000, 5, 0.02),
+    "coarse_soup": lambda: soup(300, 6, 0.4),
+    "two": lambda: W.grid_plane(1),
+    "nine": lambda: soup(9, 7, 0.3),
+}
+
+
+def rays(mesh, n, seed):
+    rng = np.random.default_rng(seed)
+    lo, hi = mesh.positions.min(0), mesh.positions.max(0)
+    o = rng.uniform(lo - 0.05, hi + 0.05, (n, 3))
+    d = rng.normal(size=(n, 3))
+    d[::3] = np.eye(3)[rng.integers(0, 3, len(d[::3]))] * rng.choice([-1, 1], (len(d[::3]), 1))  # along the axes
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    # on the mesh: at corners, on edges and inside triangles (axis-aligned rays there run in box faces)
+    p = mesh.positions[mesh.vertices[mesh.triangles, 0]].astype(np.float64)
+    w = rng.dirichlet((1, 1, 1), n)
+    w[1::4] = (0.5, 0.5, 0.0)
+    w[2::4] = (1.0, 0.0, 0.0)
+    on = (p[rng.integers(0, len(p), n)] * w[:, :, None]).sum(1)
+    o[::2] = on[::2] + rng.choice([0, 0.01, -0.01], (len(on[::2]), 1)) * d[::2]
+    o[5] = 100.0  # far outside
+    d[7, 0] = np.nan
+    o[11, 1] = np.nan
+    return o.astype(np.float32), d.astype(np.float32)
+
+
+def mapped(ctx, scene, o, d, cull, max_d):
+    n = len(o)
+    pix = np.zeros((n, 8), np.float32)
+    pix[:, 0:3], pix[:, 4:7] = o, d
+    tmap = api.TexelMap.from_host(ctx, n, 1, pix, np.zeros((n, 12), np.float32), np.arange(n))
+    coords, tidx = ctx.buffer(16 * n), ctx.buffer(4 * n)
+    api.meshmap(ctx, scene, tmap, cull, coords, tidx, max_dist=max_d)
+    return coords.download(np.float32, (n, 4)), tidx.download(np.uint32, n)
+
+
+@pytest.mark.parametrize("name", sorted(MESHES))
+@pytest.mark.parametrize("cull", [True, False])
+def test_tree_route_equals_walks(name, cull):
+    ctx = api.Context(0)
+    arrays = MESHES[name]()
+    mesh = api.Mesh(arrays)
+    mesh.compute_vertex_normals()
+    scene = api.Scene.build(ctx, mesh)
+    o, d = rays(arrays, 4099, 8)
+    for max_d, tree in ((api.FLT_MAX, api.TREE_SAH), (0.25, api.TREE_REFERENCE)):
+        scene.set_tree(tree)  # the mapping does not depend on the active tree
+        c1, t1 = mapped(ctx, scene, o, d, cull, max_d)
+        c8, t8 = mapped(ctx, scene, o, 8 * d, cull, max_d if max_d == api.FLT_MAX else max_d / 8)
+        hit = t1 != api.MISS
+        assert np.array_equal(t1, t8)
+        assert np.array_equal(c1[hit, 0], 8 * c8[hit, 0]) and np.array_equal(c1[:, 1:], c8[:, 1:])
+        assert hit.sum() > 100 or name in ("two", "nine", "flat")
+    ctx.check()
