@@ -125,27 +125,50 @@ __global__ void export_valid_kernel(const uint32_t* idx, uint32_t count, uint32_
   valid[id] = (rgb[p] | rgb[p + 1] | rgb[p + 2]) != 0;
 }
 
+// Pixels that can be a source centre: strictly inside the image with all 8
+// neighbours valid.
+__global__ void export_centre_kernel(const uint8_t* __restrict__ valid, uint32_t w, uint32_t h,
+                                     uint8_t* __restrict__ centre) {
+  const size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (p >= (size_t)w * h) return;
+  const uint32_t x = (uint32_t)(p % w), y = (uint32_t)(p / w);
+  uint32_t ok = 0;
+  if (x > 0 && y > 0 && x + 1 < w && y + 1 < h) {
+    const uint8_t *u = valid + p - w, *d = valid + p + w;
+    ok = u[-1] && u[0] && u[1] && valid[p - 1] && valid[p + 1] && d[-1] && d[0] && d[1];
+  }
+  centre[p] = (uint8_t)ok;
+}
+
 // Source centre of each uncovered pixel: the first of the reference's search
-// order (distance 1 .. max_dist - 1, 8 directions) strictly inside the image
-// with all 8 neighbours valid; -1 when none.
-__global__ void export_choice_kernel(const uint8_t* valid, uint32_t w, uint32_t h, int max_dist, int32_t* choice) {
+// order (distance 1 .. max_dist - 1, 8 directions) that can be one; -1 when
+// none.  With the 8 neighbours of every candidate checked once beforehand a
+// candidate costs one load instead of up to eight: 190 -> 137 us for both
+// kernels, 2048 x 2048 pixels, a quarter uncovered, distance 16.  Bound by the
+// latency of the dependent candidates.
+__global__ void export_choice_kernel(const uint8_t* __restrict__ valid, const uint8_t* __restrict__ centre, uint32_t w,
+                                     uint32_t h, int max_dist, int32_t* __restrict__ choice) {
   const size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (p >= (size_t)w * h) return;
   int32_t c = -1;
   if (!valid[p]) {
-    const int off[8][2] = {{1, 0}, {-1, 0}, {0, 1}, {0, -1}, {1, 1}, {1, -1}, {-1, 1}, {-1, -1}};
     const int x = (int)(p % w), y = (int)(p / w), W = (int)w, H = (int)h;
-    for (int dist = 1; dist < max_dist && c < 0; ++dist)
+    for (int dist = 1; dist < max_dist && c < 0; ++dist) {
+      // the 8 candidates' loads together, then the first that is set
+      const int dx[8] = {1, -1, 0, 0, 1, 1, -1, -1}, dy[8] = {0, 0, 1, -1, 1, -1, 1, -1};
+      uint32_t found = 0;
+#pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const int cx = x + off[k][0] * dist, cy = y + off[k][1] * dist;
-        if (!(cx > 0 && cy > 0 && cx < W - 1 && cy < H - 1)) continue;
-        bool ok = true;
-        for (int q = 0; q < 8 && ok; ++q) ok = valid[(size_t)(cx + off[q][0]) + (size_t)(cy + off[q][1]) * w] != 0;
-        if (ok) {
-          c = cy * W + cx;
-          break;
-        }
+        const int cx = x + dx[k] * dist, cy = y + dy[k] * dist;
+        if (cx >= 0 && cy >= 0 && cx < W && cy < H && centre[(size_t)cy * w + cx]) found |= 1u << k;
       }
+      if (found) {
+        const int k = __ffs(found) - 1;
+        const int kx = k < 2 ? 1 - 2 * k : (k < 4 ? 0 : (k < 6 ? 1 : -1));
+        const int ky = k < 2 ? 0 : ((k & 1) ? -1 : 1);
+        c = (y + ky * dist) * W + (x + kx * dist);
+      }
+    }
   }
   choice[p] = c;
 }
@@ -251,9 +274,10 @@ extern "C" int fk_export_image(fk_ctx* ctx, const fk_texel_map* map, const fk_bu
     if ((rc = fk_after_launch(ctx, "export scatter")) != FK_OK) return rc;
   }
   if (p->dilate > 0 && pixels > 0) {
-    uint8_t *valid = nullptr, *before = nullptr;
+    uint8_t *valid = nullptr, *before = nullptr, *centre = nullptr;
     int32_t* choice = nullptr;
     rc = fk_dev_alloc(ctx, (void**)&valid, pixels);
+    if (rc == FK_OK) rc = fk_dev_alloc(ctx, (void**)&centre, pixels);
     if (rc == FK_OK) rc = fk_dev_alloc(ctx, (void**)&choice, 4 * pixels);
     if (rc == FK_OK) rc = fk_dev_alloc(ctx, (void**)&before, 3 * pixels);
     cudaError_t e = cudaSuccess;
@@ -266,7 +290,11 @@ extern "C" int fk_export_image(fk_ctx* ctx, const fk_texel_map* map, const fk_bu
     }
     const uint32_t blocks = (uint32_t)((pixels + kThreads - 1) / kThreads);
     if (rc == FK_OK && e == cudaSuccess) {
-      export_choice_kernel<<<blocks, kThreads, 0, st>>>(valid, w, h, p->dilate, choice);
+      export_centre_kernel<<<blocks, kThreads, 0, st>>>(valid, w, h, centre);
+      rc = fk_after_launch(ctx, "export dilation centres");
+    }
+    if (rc == FK_OK && e == cudaSuccess) {
+      export_choice_kernel<<<blocks, kThreads, 0, st>>>(valid, centre, w, h, p->dilate, choice);
       rc = fk_after_launch(ctx, "export dilation sources");
     }
     if (rc == FK_OK && e == cudaSuccess) {
@@ -275,6 +303,7 @@ extern "C" int fk_export_image(fk_ctx* ctx, const fk_texel_map* map, const fk_bu
     }
     if (rc == FK_OK && e == cudaSuccess) e = cudaStreamSynchronize(st);  // before the scratch goes back
     fk_dev_free(ctx, valid);
+    fk_dev_free(ctx, centre);
     fk_dev_free(ctx, choice);
     fk_dev_free(ctx, before);
     if (rc != FK_OK) return rc;
