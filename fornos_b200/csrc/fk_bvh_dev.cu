@@ -22,6 +22,7 @@
 
 #include "fk_bvh_rules.h"
 #include "fk_internal.h"
+#include "fk_sah_rules.h"
 
 namespace fk {
 namespace {
@@ -702,6 +703,61 @@ __global__ void bvh_corners_below_kernel(const float4* __restrict__ p, uint32_t 
   }
 }
 
+// The scene layout of a device-built tree's nodes, as fk_layout.cpp makes it
+// of an uploaded array: 2-wide records of the inner nodes in preorder, leaf
+// indices in order, levels, and whether all coordinates admit the filtered box
+// tests (words[1] bit 0 clear) and the rebuilt tree (bit 1 clear).  One thread a
+// node walks down to it from the root; with p the ancestors whose left subtree
+// holds it, (i + p) / 2 inner nodes and (i - p) / 2 leaves come before node i of
+// a full binary tree, so no scan is needed.  663k nodes (2.1M triangles): the
+// nodes' way to the host, its layout of them and the records' way back took
+// 17 of fk_scene_build's 45.6 ms, this kernel takes under 0.08 ms (bound by the
+// walk's dependent loads).
+__global__ void bvh_layout_kernel(const float4* __restrict__ lo, const float4* __restrict__ hi,
+                                  const uint32_t* __restrict__ jump, uint32_t nn, float4* __restrict__ wide,
+                                  uint32_t* __restrict__ leaf_ids, uint32_t* __restrict__ words) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t level = 1, bad = 0;
+  if (i < nn) {
+    uint32_t p = 0;
+    for (uint32_t c = 0; c != i; ++level) {
+      const uint32_t right = __ldg(jump + c + 1);
+      const bool left = i < right;
+      p += left;
+      c = left ? c + 1 : right;
+    }
+    const float4 L = lo[i], H = hi[i];
+    const bool leaf = __ldg(jump + i) == i + 1;
+    for (int q = 0; q < 3; ++q) {
+      const float l = comp(L, q), h = comp(H, q);
+      if (!(fabsf(l) < 16777216.0f && fabsf(h) < 16777216.0f && l <= h)) bad |= 1u;
+      if (leaf && !(sah::coord_ok(l) && sah::coord_ok(h))) bad |= 2u;
+    }
+    if (leaf) {
+      leaf_ids[(i - p) / 2] = i;
+    } else {
+      const uint32_t a = i + 1, b = __ldg(jump + a);
+      const float4 AL = lo[a], AH = hi[a], BL = lo[b], BH = hi[b];
+      const bool la = b == a + 1, lb = __ldg(jump + b) == b + 1;
+      const int32_t ra = la ? -(int32_t)a - 1 : (int32_t)((a + p + 1) / 2);
+      const int32_t rb = lb ? -(int32_t)b - 1 : (int32_t)((b + p) / 2);
+      const int32_t ca = la ? (int32_t)((__float_as_uint(AH.w) - __float_as_uint(AL.w)) / 3) : 0;
+      const int32_t cb = lb ? (int32_t)((__float_as_uint(BH.w) - __float_as_uint(BL.w)) / 3) : 0;
+      float4* w = wide + 4 * (size_t)((i + p) / 2);
+      w[0] = make_float4(AL.x, AH.x, AL.y, AH.y);
+      w[1] = make_float4(BL.x, BH.x, BL.y, BH.y);
+      w[2] = make_float4(AL.z, AH.z, BL.z, BH.z);
+      w[3] = make_float4(__int_as_float(ra), __int_as_float(rb), __int_as_float(ca), __int_as_float(cb));
+    }
+  }
+  level = __reduce_max_sync(0xFFFFFFFFu, level);
+  bad = __reduce_or_sync(0xFFFFFFFFu, bad);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(words, level);
+    if (bad) atomicOr(words + 1, bad);
+  }
+}
+
 // ------------------------------------------------------------ host side
 struct HNode {
   float c[3], s[3];
@@ -746,6 +802,38 @@ int corners_below(fk_ctx* ctx, const float4* p, uint32_t n, float lim, bool* ok)
   if (rc != FK_OK) return rc;
   if (e != cudaSuccess) return fk_cuda_fail(ctx, e, "corner bound");
   *ok = h == 0;
+  return FK_OK;
+}
+
+int layout_bvh_device(fk_ctx* ctx, const DevBvh& d, DevLayout* out) {
+  *out = DevLayout{};
+  const uint32_t nn = d.node_count;
+  out->leaves = nn / 2 + 1;  // a full binary tree
+  out->wide_count = nn / 2;
+  uint32_t* words = nullptr;
+  uint32_t h[2] = {0, 0};
+  int rc = fk_dev_alloc(ctx, (void**)&words, 8);
+  if (rc == FK_OK) rc = fk_dev_alloc(ctx, (void**)&out->leaf_ids, 4 * (size_t)out->leaves);
+  if (rc == FK_OK && out->wide_count) rc = fk_dev_alloc(ctx, (void**)&out->wide, 4 * sizeof(float4) * (size_t)out->wide_count);
+  cudaError_t e = cudaSuccess;
+  if (rc == FK_OK) e = cudaMemsetAsync(words, 0, 8, ctx->stream);
+  if (rc == FK_OK && e == cudaSuccess) {
+    bvh_layout_kernel<<<(nn + 255) / 256, 256, 0, ctx->stream>>>(d.lo, d.hi, d.jump, nn, out->wide, out->leaf_ids, words);
+    rc = fk_after_launch(ctx, "bvh_layout_kernel");
+  }
+  if (rc == FK_OK && e == cudaSuccess) e = cudaMemcpyAsync(h, words, 8, cudaMemcpyDeviceToHost, ctx->stream);
+  if (rc == FK_OK && e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  fk_dev_free(ctx, words);
+  if (rc == FK_OK && e != cudaSuccess) rc = fk_cuda_fail(ctx, e, "device BVH layout");
+  if (rc != FK_OK) {
+    fk_dev_free(ctx, out->leaf_ids);
+    fk_dev_free(ctx, out->wide);
+    *out = DevLayout{};
+    return rc;
+  }
+  out->depth = h[0];
+  out->coords_ok = !(h[1] & 1u);
+  out->sah_ok = !(h[1] & 2u);
   return FK_OK;
 }
 

@@ -301,37 +301,53 @@ void* fk_buf_device_ptr(const fk_buf* b) { return b ? b->ptr : nullptr; }
 // ------------------------------------------------------------------ scene
 }  // extern "C"
 
-// Scene from a flattened node array: host corner arrays (fk_scene_upload), or
-// the device build's arrays, which the scene adopts (`dev`: nodes, corners).
+// Scene from a flattened node array and host corner arrays (fk_scene_upload),
+// or from a device build's arrays, which the scene adopts (`dev`; nodes, pos4
+// and nrm4 are null then).
 static int scene_create(fk_ctx* ctx, const fk_bvh_node* nodes, uint32_t nn, const float* pos4, const float* nrm4,
                         uint32_t nc, fk::DevBvh* dev, fk_scene** out) {
-  if (!ctx || !out || !nodes || (!dev && (!pos4 || !nrm4)) || nn == 0 || nc == 0 || nc % 3 != 0)
+  if (!ctx || !out || (!dev && (!nodes || !pos4 || !nrm4)) || nn == 0 || nc == 0 || nc % 3 != 0)
     return fk_fail(ctx, FK_ERR_INVALID, "fk_scene_upload: empty or malformed scene");
-  // Check the skip-pointer structure so no kernel can walk outside it, and
-  // lay out the device arrays (fk_layout.cpp, over host threads) in the
-  // context's pinned staging, once the previous upload's copies from it are
-  // done.
-  const size_t stage_need = fk::layout_bytes(nn);
-  if (ctx->stage_done) FK_CUDA(ctx, cudaEventSynchronize(ctx->stage_done));
-  if (ctx->stage_bytes < stage_need) {
-    if (ctx->stage) FK_CUDA(ctx, cudaFreeHost(ctx->stage));
-    ctx->stage = nullptr;
-    ctx->stage_bytes = 0;
-    if (cudaMallocHost(&ctx->stage, stage_need) != cudaSuccess) {
-      cudaGetLastError();
-      ctx->stage = nullptr;
-      return fk_fail(ctx, FK_ERR_NOMEM, "fk_scene_upload: pinned staging of " + std::to_string(stage_need) + " bytes");
-    }
-    ctx->stage_bytes = stage_need;
-  }
   fk::NodeLayout lay;
-  const std::string bad = fk::layout_nodes(nodes, nn, nc, ctx->stage, lay);
-  if (!bad.empty()) return fk_fail(ctx, FK_ERR_INVALID, bad);
-  const uint32_t leaves = lay.leaves, nw = lay.wide_count, maxd = lay.depth;
-  const bool sah_ok = lay.sah_ok;  // leaf boxes within the rebuilt tree's coordinate range
-  const std::vector<uint32_t>& leaf_ids = lay.leaf_ids;
+  fk::DevLayout dlay;
+  if (dev) {
+    const int rc = fk::layout_bvh_device(ctx, *dev, &dlay);
+    if (rc != FK_OK) return rc;
+  } else {
+    // Check the skip-pointer structure so no kernel can walk outside it, and
+    // lay out the device arrays (fk_layout.cpp, over host threads) in the
+    // context's pinned staging, once the previous upload's copies from it are
+    // done.
+    const size_t stage_need = fk::layout_bytes(nn);
+    if (ctx->stage_done) FK_CUDA(ctx, cudaEventSynchronize(ctx->stage_done));
+    if (ctx->stage_bytes < stage_need) {
+      if (ctx->stage) FK_CUDA(ctx, cudaFreeHost(ctx->stage));
+      ctx->stage = nullptr;
+      ctx->stage_bytes = 0;
+      if (cudaMallocHost(&ctx->stage, stage_need) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->stage = nullptr;
+        return fk_fail(ctx, FK_ERR_NOMEM, "fk_scene_upload: pinned staging of " + std::to_string(stage_need) + " bytes");
+      }
+      ctx->stage_bytes = stage_need;
+    }
+    const std::string bad = fk::layout_nodes(nodes, nn, nc, ctx->stage, lay);
+    if (!bad.empty()) return fk_fail(ctx, FK_ERR_INVALID, bad);
+  }
+  const uint32_t leaves = dev ? dlay.leaves : lay.leaves, nw = dev ? dlay.wide_count : lay.wide_count;
+  const uint32_t maxd = dev ? dlay.depth : lay.depth;
+  const bool sah_ok = dev ? dlay.sah_ok : lay.sah_ok;  // leaf boxes within the rebuilt tree's coordinate range
+  const bool coords_ok = dev ? dlay.coords_ok : lay.coords_ok;
+  auto drop_layout = [&] {
+    fk_dev_free(ctx, dlay.leaf_ids);
+    fk_dev_free(ctx, dlay.wide);
+    dlay = fk::DevLayout{};
+  };
   fk_scene* s = new (std::nothrow) fk_scene();
-  if (!s) return FK_ERR_NOMEM;
+  if (!s) {
+    drop_layout();
+    return FK_ERR_NOMEM;
+  }
   s->ctx = ctx;
   s->node_count = nn;
   s->corner_count = nc;
@@ -341,19 +357,20 @@ static int scene_create(fk_ctx* ctx, const fk_bvh_node* nodes, uint32_t nn, cons
   s->wide_count = nw;
   s->wide4_count = 0;  // the 4-wide layout is built on first use (fk::ensure_wide4)
   s->depth4 = 0;
-  s->root_is_leaf = nodes[0].jump == 1;
+  s->root_is_leaf = nn == 1;
   // The filtered box tests assume |box - origin| < 2^26; ray origins lie on
   // the scene's triangles, so box and corner coordinates below 2^24 suffice.
   // The conservative inner test also takes each box's faces in order.
   {
     const float lim = 16777216.0f;
-    bool ok = lay.coords_ok;
+    bool ok = coords_ok;
     if (!dev) {
       // the corners are checked on the device once uploaded (below)
     } else if (ok) {
       bool below = false;
       const int rc = fk::corners_below(ctx, dev->pos4, nc, lim, &below);
       if (rc != FK_OK) {
+        drop_layout();
         delete s;
         return rc;
       }
@@ -379,16 +396,17 @@ static int scene_create(fk_ctx* ctx, const fk_bvh_node* nodes, uint32_t nn, cons
     s->pos4 = dev->pos4;
     s->nrm4 = dev->nrm4;
     *dev = fk::DevBvh{};
-    s->bytes += 2 * nb + sizeof(uint32_t) * nn + 2 * cb;
+    s->wide = dlay.wide;
+    dlay.wide = nullptr;
+    s->bytes += 2 * nb + sizeof(uint32_t) * nn + 2 * cb + sizeof(float4) * 4 * (size_t)nw;
   } else {
     up((void**)&s->node_lo, lay.lo, nb);
     up((void**)&s->node_hi, lay.hi, nb);
     up((void**)&s->node_jump, lay.jump, sizeof(uint32_t) * nn);
     up((void**)&s->pos4, pos4, cb);
     up((void**)&s->nrm4, nrm4, cb);
-  }
-  up((void**)&s->wide, lay.wide, sizeof(float4) * 4 * (size_t)nw);
-  {  // the copies above read the staging: the next upload waits for them
+    up((void**)&s->wide, lay.wide, sizeof(float4) * 4 * (size_t)nw);
+    // the copies above read the staging: the next upload waits for them
     cudaError_t e = cudaSuccess;
     if (!ctx->stage_done) e = cudaEventCreateWithFlags(&ctx->stage_done, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventRecord(ctx->stage_done, ctx->stream);
@@ -412,7 +430,8 @@ static int scene_create(fk_ctx* ctx, const fk_bvh_node* nodes, uint32_t nn, cons
   if (rc == FK_OK && nw > 0 && sah_ok) {
     float4* sw = nullptr;
     uint32_t sdepth = 0;
-    rc = fk::build_sah_device(ctx, s->node_lo, s->node_hi, leaf_ids, &sw, &sdepth);
+    rc = fk::build_sah_device(ctx, s->node_lo, s->node_hi, dev ? dlay.leaf_ids : lay.leaf_ids.data(), leaves, &sw,
+                              &sdepth);
     if (rc == FK_OK && sw) {
       s->tree_wide[FK_TREE_SAH] = sw;
       s->tree_count[FK_TREE_SAH] = leaves - 1;
@@ -420,6 +439,7 @@ static int scene_create(fk_ctx* ctx, const fk_bvh_node* nodes, uint32_t nn, cons
       s->bytes += sizeof(float4) * 4 * (size_t)(leaves - 1);
     }
   }
+  fk_dev_free(ctx, dlay.leaf_ids);  // in stream order, behind the build that read it
   if (rc == FK_OK) {
     rc = fk_dev_alloc(ctx, (void**)&s->tri_rec, 4 * sizeof(float4) * (size_t)(nc / 3));
     s->bytes += 4 * sizeof(float4) * (size_t)(nc / 3);
@@ -539,9 +559,7 @@ int fk_scene_build(fk_ctx* ctx, const fk_mesh* mesh, uint32_t max_tris, uint32_t
     dev_free(ctx, d);
     return fk_fail(ctx, FK_ERR_INVALID, "fk_scene_build: the mesh has no triangles");
   }
-  std::vector<fk_bvh_node> v;
-  rc = dev_nodes(ctx, d, v);
-  if (rc == FK_OK) rc = scene_create(ctx, v.data(), d.node_count, nullptr, nullptr, d.corner_count, &d, out);
+  rc = scene_create(ctx, nullptr, d.node_count, nullptr, nullptr, d.corner_count, &d, out);
   dev_free(ctx, d);  // nothing left after a successful adoption
   return rc;
 }

@@ -199,14 +199,23 @@ struct DevBvh {
   uint32_t node_count = 0, corner_count = 0, triangle_count = 0;
 };
 int build_bvh_device(fk_ctx* ctx, const fk_mesh* mesh, uint32_t max_tris, uint32_t max_depth, DevBvh* out);
+// The scene layout of a device-built tree (fk_layout.h's NodeLayout, on the
+// device): records and leaf indices are the caller's to free.
+struct DevLayout {
+  float4* wide = nullptr;
+  uint32_t* leaf_ids = nullptr;
+  uint32_t leaves = 0, wide_count = 0, depth = 0;
+  bool coords_ok = false, sah_ok = false;
+};
+int layout_bvh_device(fk_ctx* ctx, const DevBvh& d, DevLayout* out);
 // *ok: every coordinate of the n corners is below lim in magnitude.
 int corners_below(fk_ctx* ctx, const float4* p, uint32_t n, float lim, bool* ok);
 
 // The same tree built on the device (fk_sah.cu) from the scene's node boxes
-// and its leaves' flattened indices (ascending): *wide gets 4 (L - 1) float4
+// and its leaves' flattened indices (ascending, in host or device memory): *wide gets 4 (L - 1) float4
 // records, or stays null when the tree would be deeper than
 // kMaxOrderedDepth (*depth then exceeds it); depth 1 for a single leaf.
-int build_sah_device(fk_ctx* ctx, const float4* node_lo, const float4* node_hi, const std::vector<uint32_t>& leaves,
+int build_sah_device(fk_ctx* ctx, const float4* node_lo, const float4* node_hi, const uint32_t* leaves, uint32_t leaf_count,
                      float4** wide, uint32_t* depth);
 // The scene's 4-wide layout for its active tree, built on first use.
 int ensure_wide4(fk_ctx* ctx, fk_scene* s);

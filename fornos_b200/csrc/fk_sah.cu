@@ -526,11 +526,10 @@ T* carve(char*& p, size_t count) {
 
 }  // namespace
 
-int build_sah_device(fk_ctx* ctx, const float4* lo, const float4* hi, const std::vector<uint32_t>& leaves,
+int build_sah_device(fk_ctx* ctx, const float4* lo, const float4* hi, const uint32_t* leaves, uint32_t L,
                      float4** out_wide, uint32_t* out_depth) {
   *out_wide = nullptr;
   *out_depth = 0;
-  const uint32_t L = (uint32_t)leaves.size();
   if (L < 2) {
     *out_depth = 1;
     return FK_OK;
@@ -582,7 +581,7 @@ int build_sah_device(fk_ctx* ctx, const float4* lo, const float4* hi, const std:
     if (e_ != cudaSuccess) return fail(fk_cuda_fail(ctx, e_, #call)); \
   } while (0)
   cudaStream_t st = ctx->stream;
-  FK_SAH_TRY(cudaMemcpyAsync(perm[0], leaves.data(), 4 * (size_t)L, cudaMemcpyHostToDevice, st));
+  FK_SAH_TRY(cudaMemcpyAsync(perm[0], leaves, 4 * (size_t)L, cudaMemcpyDefault, st));
   FK_SAH_TRY(cudaMemsetAsync(words, 0, 8, st));
 
   std::vector<Task> cur, small;
