@@ -169,13 +169,25 @@ int fk_batch_create(fk_ctx* ctx, const fk_batch_job* jobs, uint32_t njobs, int k
   if (njobs > fk::kMaxBatchJobs)
     return fk_fail(ctx, FK_ERR_INVALID, "fk_batch_create: at most " + std::to_string(fk::kMaxBatchJobs) + " jobs");
   if (kind < FK_AO || kind > FK_AO_BN) return fk_fail(ctx, FK_ERR_INVALID, "fk_batch_create: unknown kind");
+  // the jobs that share launches first, in the order given, so that their rays
+  // lie end to end: one launch then takes them all, where a solo job between two
+  // of them would cut it (three shared launches instead of one, and a launch's
+  // tail each: 3.52 -> 3.40 ms for 16 small jobs)
+  std::vector<fk_batch_job> ordered(jobs, jobs + njobs);
+  std::vector<uint32_t> given(njobs);
+  for (uint32_t i = 0; i < njobs; ++i) given[i] = i;
+  std::stable_partition(given.begin(), given.end(), [&](uint32_t i) {
+    return (unsigned long long)jobs[i].texel_count * jobs[i].params.sample_count < kSoloRays;
+  });
+  for (uint32_t i = 0; i < njobs; ++i) ordered[i] = jobs[given[i]];
+  jobs = ordered.data();
   std::vector<fk::BatchJobDev> table(njobs);
   unsigned long long rays = 0;
   uint64_t texels = 0, nodes = 0, corners = 0, recs2 = 0, recs4 = 0;
   for (uint32_t i = 0; i < njobs; ++i) {
     const fk_batch_job& J = jobs[i];
     const uint64_t n = J.texel_count;
-    const std::string who = "fk_batch_create: job " + std::to_string(i);
+    const std::string who = "fk_batch_create: job " + std::to_string(given[i]);
     if (!J.scene || !ctx->scenes.count(const_cast<fk_scene*>(J.scene)))
       return fk_fail(ctx, FK_ERR_INVALID, who + " has no scene of this context");
     if (J.params.sample_count == 0 || J.params.perm_count == 0)
