@@ -55,6 +55,15 @@ static SceneDev dev_of(const fk_scene* s) {
 
 __device__ __forceinline__ uint32_t as_u32(float f) { return __float_as_uint(f); }
 
+// Two consecutive float4 at a 32-byte boundary by one 256-bit load.  In the inner
+// visit two of these replace four 128-bit loads: thickness of 500 x 500 texels at
+// 100 spp 8.45 -> 8.15 ms, AO + BN 21.24 -> 21.13 ms (2.1M triangles).
+__device__ __forceinline__ void ldg2(const float4* p, float4& a, float4& b) {
+  asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
+
 // ------------------------------------------------------------------ records
 // Per triangle (a, b, c): n = normalize(cross(b - a, c - a)) and dot(a, n) as
 // Shaders/ao_step1.comp:73-77 computes them, plus the barycentric terms of
@@ -747,7 +756,8 @@ __device__ __forceinline__ bool inner_visit(const SceneDev& s, const RayPre& rp,
     w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3];
   } else {
     const float4* w = s.wide + 4 * (size_t)st.cur;
-    w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2), w3 = __ldg(w + 3);
+    ldg2(w, w0, w1);
+    ldg2(w + 2, w2, w3);
   }
   float d0, d1;
   const bool h0 = child_maybe<FILTER, S>(rp, ray, mk3(w0.x, w0.z, w2.x), mk3(w0.y, w0.w, w2.y), thr, d0);
