@@ -64,10 +64,27 @@ __device__ __forceinline__ float gelu(float z, float& dz) {
   return (0.5f * z) * (1.0f + th);
 }
 
-// The same value without the derivative.
-__device__ __forceinline__ float gelu_value(float z) {
-  const float u = 0.7978845608028654f * (z + 0.044715f * ((z * z) * z));
-  return (0.5f * z) * (1.0f + tanhf(u));
+// Two at once: the products and sums as packed pairs (the same roundings, half
+// the instructions), tanhf for each.
+__device__ __forceinline__ uint64_t pair(float a, float b) {
+  return (uint64_t)__float_as_uint(b) << 32 | __float_as_uint(a);
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float2 gelu_pair(uint64_t z) {
+  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
+  const uint64_t u = mul2(pair(k0, k0), add2(z, mul2(pair(k1, k1), mul2(mul2(z, z), z))));
+  const uint64_t th = pair(tanhf(__uint_as_float((uint32_t)u)), tanhf(__uint_as_float((uint32_t)(u >> 32))));
+  const uint64_t g = mul2(mul2(pair(0.5f, 0.5f), z), add2(pair(1.0f, 1.0f), th));
+  return make_float2(__uint_as_float((uint32_t)g), __uint_as_float((uint32_t)(g >> 32)));
 }
 
 // Octahedral encoding of a direction (zero or non-finite vectors map to 0).
@@ -90,11 +107,11 @@ __device__ __forceinline__ float clamp4(float v) { return fminf(fmaxf(v, -4.0f),
 // position and spacing.
 struct Centre {
   int x, y;
-  float px, py, pz, spacing;
+  float px, py, pz, spacing, inv;  // inv: 1 / spacing where `over_spacing` may use it, else 0
 };
 __device__ __forceinline__ Centre centre_of(const float4* __restrict__ f1, const float4* __restrict__ f2, uint32_t w,
                                             uint32_t p) {
-  Centre c = {0, 0, 0.0f, 0.0f, 0.0f, 0.0f};
+  Centre c = {0, 0, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
   if (p == kNoTexel) return c;
   const float4 b = __ldg(f1 + p);
   c.y = (int)(p / w);
@@ -103,12 +120,26 @@ __device__ __forceinline__ Centre centre_of(const float4* __restrict__ f1, const
   c.py = b.y;
   c.pz = b.z;
   c.spacing = __ldg(f2 + p).z;
+  c.inv = c.spacing > 8.67361738e-19f && c.spacing < 1.15292150e18f ? __frcp_rn(c.spacing) : 0.0f;  // 2^-60, 2^60
   return c;
+}
+
+// v / spacing by the centre's reciprocal and one residual correction (P.
+// Markstein, 1990): correctly rounded but for quotients next to a midpoint of
+// two floats, far below the bf16 rounding of what it feeds.  A texel divides 75
+// times by the same spacing.  Outside the reciprocal's range, or for a quotient
+// that is not finite, the division itself.
+__device__ __forceinline__ float over_spacing(float v, const Centre& c) {
+  const float q = v * c.inv;
+  const float r = __fmaf_rn(__fmaf_rn(-q, c.spacing, v), c.inv, q);
+  return c.inv > 0.0f && fabsf(r) < 1.0e30f ? r : v / c.spacing;
 }
 
 // The 10 features of neighbour j (< 25, row-major over the 5 x 5 window) of
 // the texel at pixel p with centre terms c; zeros outside the texture, without
-// a mapping hit, or for p = kNoTexel.
+// a mapping hit, or for p = kNoTexel.  EXACT: IEEE divisions (the rows that a
+// caller keeps); else over_spacing.
+template <bool EXACT>
 __device__ __forceinline__ void neighbour_features(const float4* __restrict__ f0, const float4* __restrict__ f1,
                                                    const float4* __restrict__ f2, uint32_t w, uint32_t h, uint32_t p,
                                                    const Centre& c, int j, float (&v)[10]) {
@@ -124,9 +155,9 @@ __device__ __forceinline__ void neighbour_features(const float4* __restrict__ f0
   v[1] = a.y;
   v[2] = a.z;
   if (c.spacing > 0.0f) {
-    v[3] = clamp4((b.x - c.px) / c.spacing);
-    v[4] = clamp4((b.y - c.py) / c.spacing);
-    v[5] = clamp4((b.z - c.pz) / c.spacing);
+    v[3] = clamp4(EXACT ? (b.x - c.px) / c.spacing : over_spacing(b.x - c.px, c));
+    v[4] = clamp4(EXACT ? (b.y - c.py) / c.spacing : over_spacing(b.y - c.py, c));
+    v[5] = clamp4(EXACT ? (b.z - c.pz) / c.spacing : over_spacing(b.z - c.pz, c));
   }
   v[6] = n.x;
   v[7] = n.y;
@@ -141,7 +172,7 @@ __device__ __forceinline__ void assemble_row(const float4* __restrict__ f0, cons
                                              int lane, uint32_t* dst) {
   if (lane < 25) {
     float v[10];
-    neighbour_features(f0, f1, f2, w, h, p, centre_of(f1, f2, w, p), lane, v);
+    neighbour_features<true>(f0, f1, f2, w, h, p, centre_of(f1, f2, w, p), lane, v);
 #pragma unroll
     for (int k = 0; k < 5; ++k) dst[5 * lane + k] = pack2(v[2 * k], v[2 * k + 1]);
   } else if (lane == 25) {
@@ -882,9 +913,9 @@ __device__ __forceinline__ void hidden_epilogue(uint32_t taddr, uint32_t c0, con
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const uint32_t c = c0 + 8 * h + 2 * e;
-      const float a0 = gelu_value(v[8 * h + 2 * e] + __ldg(bias + c));
-      const float a1 = gelu_value(v[8 * h + 2 * e + 1] + __ldg(bias + c + 1));
-      w4[e] = pack2(a0, a1);
+      const float2 b = __ldg((const float2*)(bias + c));
+      const float2 g = gelu_pair(add2(pair(v[8 * h + 2 * e], v[8 * h + 2 * e + 1]), pair(b.x, b.y)));
+      w4[e] = pack2(g.x, g.y);
     }
     *(uint4*)(dst + core_off(row, c0 + 8 * h, 64)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
   }
@@ -897,7 +928,9 @@ __device__ __forceinline__ void hidden_epilogue(uint32_t taddr, uint32_t c0, con
 // the 16-byte operand stores hit all banks) and every fourth neighbour.  One
 // warp per row with a lane per neighbour, scattered loads and 4-byte stores and
 // one CTA per SM took 593 us for a 1024 x 1024 map (750k texels); this takes
-// 288 us (issue 57 % active, 7.4k thread instructions a texel, tanhf most of them).
+// 288 us, and 274 us with the GELUs' products and sums in packed pairs and one
+// reciprocal a texel for its 75 quotients (issue 57 % active before those two,
+// 7.4k thread instructions a texel, tanhf most of them).
 __global__ void __launch_bounds__(tc::kThreads, tc::kCtasPerSm) dn_apply_tc_kernel(ApplyArgs a, int* status) {
   extern __shared__ __align__(128) unsigned char sm[];
   const uint32_t sb = (uint32_t)__cvta_generic_to_shared(sm);
@@ -968,7 +1001,7 @@ __global__ void __launch_bounds__(tc::kThreads, tc::kCtasPerSm) dn_apply_tc_kern
 #pragma unroll 2
       for (uint32_t j = part; j < 25; j += 4) {
         float v[10];
-        neighbour_features(a.f0, a.f1, a.f2, a.w, a.h, px, c, (int)j, v);
+        neighbour_features<false>(a.f0, a.f1, a.f2, a.w, a.h, px, c, (int)j, v);
         *(uint4*)(sm + tc::kA1 + tc::core_off(r, 8 * j, 256)) =
             make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
         *(uint32_t*)(sm + tc::kA1 + tc::core_off(r, 200 + 2 * j, 256)) = pack2(v[8], v[9]);

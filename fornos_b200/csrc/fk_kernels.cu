@@ -2082,6 +2082,7 @@ __device__ float walk_twoside(const SceneDev& s, f3 o, f3 d, float mint, uint32_
 // times a node and visit hundreds of the reference tree's nodes a ray.
 // 2048 x 2048 texels on the 2.1M-triangle heightfield: 4.71 -> 1.03 ms; 128 x 128 texels
 // on a 9k-triangle sphere: 283 -> 59 us.
+constexpr uint32_t kMaxChain = 1u << 15;  // a level is two steps at most; the builds stop at 8192 levels
 __global__ void map_pad_kernel(const float4* __restrict__ lo, const float4* __restrict__ hi,
                                const uint32_t* __restrict__ jump, const float4* __restrict__ pos4,
                                const float4* __restrict__ rec, uint32_t nodes, uint32_t* __restrict__ pad,
@@ -2099,7 +2100,8 @@ __global__ void map_pad_kernel(const float4* __restrict__ lo, const float4* __re
     };
     if (as_u32(L.w) < as_u32(H.w)) {  // a leaf: down to it from the root
       f3 cl = xyz(L), ch = xyz(H);
-      for (uint32_t c = 0; c < i;) {
+      uint32_t steps = 0;
+      for (uint32_t c = 0; c < i && ++steps <= kMaxChain;) {
         if (jump[c] <= i) {
           c = jump[c];
         } else {
@@ -2108,6 +2110,7 @@ __global__ void map_pad_kernel(const float4* __restrict__ lo, const float4* __re
           ++c;
         }
       }
+      if (steps > kMaxChain) p = inf;  // an uploaded tree of extreme depth: the walks
       chain[2 * (size_t)i] = make_float4(cl.x, cl.y, cl.z, 0.0f);
       chain[2 * (size_t)i + 1] = make_float4(ch.x, ch.y, ch.z, 0.0f);
     }
@@ -2133,6 +2136,7 @@ __global__ void map_pad_kernel(const float4* __restrict__ lo, const float4* __re
 }
 
 int launch_map_pad(fk_ctx* ctx, fk_scene* s) {
+  if (!s->tree_wide[FK_TREE_SAH]) return FK_OK;  // nothing reads it (launch_meshmap)
   const cudaError_t e = cudaMemsetAsync(s->map_pad, 0, sizeof(float), ctx->stream);
   if (e != cudaSuccess) return fk_cuda_fail(ctx, e, "mapping bound");
   map_pad_kernel<<<(s->node_count + 255) / 256, 256, 0, ctx->stream>>>(s->node_lo, s->node_hi, s->node_jump, s->pos4,
