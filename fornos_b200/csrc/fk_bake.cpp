@@ -20,6 +20,8 @@ struct Scoped {
     if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
     for (fk_buf* b : bufs) fk_buf_release(ctx, b);  // used on the context's stream only
     if (scene) fk_scene_free(ctx, scene);
+    // the caller's texel rows may still be on their way up (a scene that was refused): not after the return
+    if (map) cudaStreamSynchronize(ctx->stream);
     if (map) fk_texel_map_free(ctx, map);
   }
   int alloc(size_t bytes, fk_buf** out) {

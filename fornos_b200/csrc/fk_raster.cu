@@ -302,8 +302,10 @@ extern "C" int fk_raster_uv(fk_ctx* ctx, const fk_mesh* m, const fk_mesh* dirs, 
   if (rc == FK_OK) rc = fk_dev_alloc(ctx, (void**)&counts, 4 * (size_t)(tiles + 1));
   fk_texel_map* map = nullptr;
   uint32_t count = 0;
+  // freed in stream order behind the kernels that read them (fk_dev_free); the
+  // copy from `tris` was over at the count's read-back, or waits here on failure
   auto cleanup = [&]() {
-    cudaStreamSynchronize(ctx->stream);
+    if (rc != FK_OK) cudaStreamSynchronize(ctx->stream);
     fk_dev_free(ctx, dtris);
     fk_dev_free(ctx, owner);
     fk_dev_free(ctx, counts);
