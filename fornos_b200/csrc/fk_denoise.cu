@@ -791,8 +791,8 @@ __global__ void __launch_bounds__(256, 2) dn_apply_kernel(ApplyArgs a) {
 }
 
 // ------------------------------------------------------------------ inference on tcgen05
-// The same network on sm_100's fifth-generation tensor cores: a CTA of one
-// warpgroup (128 threads) owns a 128-texel tile; the tile's input rows and the
+// The same network on sm_100's fifth-generation tensor cores: a CTA of
+// 16 warps owns a 128-texel tile; the tile's input rows and the
 // weights sit in shared memory in the no-swizzle K-major core-matrix layout
 // (8 rows x 16 bytes per core matrix, core matrices 128 bytes apart along K
 // and SBO bytes apart along the rows), one elected thread issues

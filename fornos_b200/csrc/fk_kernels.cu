@@ -963,9 +963,10 @@ __device__ __forceinline__ bool leaf_phase_warp(const SceneDev& s, const RayPre&
 // 2.1M-triangle heightfield, of which 18.5 hold its own origin, at 10 to 11 of
 // a warp's 32 lanes a visit; here the freshly filled lanes test one sibling a
 // level together, and 15.3 visits are left.  The kernel is bound by issue and
-// load latency, so time follows the visits: AO + BN of 1024 x 1024 texels at 256
-// spp on that heightfield 120.0 -> 105.4 ms, AO of 512 x 512 texels at 64 spp on
-// the 261k-triangle sphere 5.59 -> 4.74 ms.
+// load latency, so time follows the visits: this alone took AO + BN of 1024 x
+// 1024 texels at 256 spp on that heightfield from 120.0 to 105.4 ms (87.0 with the
+// leaf phase and lane state below) and AO of 512 x 512 texels at 64 spp on the
+// 261k-triangle sphere from 5.59 to 4.74 ms (3.94).
 template <bool COUNT, bool FILTER, int S>
 __device__ __forceinline__ void path_start(const float4* __restrict__ wide, const RayPre& rp, const float* ray,
                                            int32_t root, uint64_t path, float hi, OState& st, int32_t* stk,

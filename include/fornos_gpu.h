@@ -227,9 +227,11 @@ int fk_scene_get_info(const fk_scene* scene, fk_scene_info* out);
  * Leaves, leaf boxes and the skip-pointer walk are untouched, and the outcome
  * is that of any inner tree over these leaves (an inner box only prunes what
  * its leaves' own tests reject), so results stay within the ordered
- * traversal's bar.  Both trees stay resident.  The rebuilt tree is not built
- * when a leaf box coordinate is not finite or not below 1e30 in magnitude, nor
- * kept when it is deeper than 48 levels. */
+ * traversal's bar.  Both trees stay resident; choosing the reference's for the
+ * first time allocates 8 bytes per triangle (where a ray starts in it).  Mesh
+ * mapping does not depend on the choice.  The rebuilt tree is not built when a
+ * leaf box coordinate is not finite or not below 1e30 in magnitude, nor kept
+ * when it is deeper than 48 levels. */
 #define FK_TREE_REFERENCE 0
 #define FK_TREE_SAH 1
 int fk_scene_set_tree(fk_scene* scene, int tree);
