@@ -541,7 +541,7 @@ int launch_hemisphere(fk_ctx* ctx, const fk_scene* s, const HemiLaunch& h) {
   a.out1 = h.out1;
   a.hits0 = h.hits0;
   a.hits1 = h.hits1;
-  a.queue = fk_take_counter(ctx);
+  a.queue = nullptr;  // the static schedule's, taken below; a dynamic launch takes its own
   a.status = ctx->status;
   a.tally = h.tally;
   a.ids = h.ids;
@@ -554,6 +554,7 @@ int launch_hemisphere(fk_ctx* ctx, const fk_scene* s, const HemiLaunch& h) {
   if (trav == FK_TRAVERSE_ORDERED4 && s->depth4 > kMaxOrdered4Depth)
     return fk_fail(ctx, FK_ERR_INVALID, "4-wide traversal needs a 4-wide depth <= 21; use FK_TRAVERSE_ORDERED");
   if (sched == 0) sched = FK_SCHEDULE_DYNAMIC;
+  if (sched != FK_SCHEDULE_DYNAMIC) a.queue = fk_take_counter(ctx);
   if (h.ids && sched != FK_SCHEDULE_DYNAMIC)
     return fk_fail(ctx, FK_ERR_UNSUPPORTED, "texel lists run on the dynamic schedule only");
   if (trav == FK_TRAVERSE_ORDERED4 && sched != FK_SCHEDULE_DYNAMIC)
