@@ -63,7 +63,7 @@ struct fk_batch {
   fk_tuning tuning = {8, 8, 0, 0, 0, FK_L2_NONE, 256, 64};
   // the jobs' scenes laid end to end (fk::BatchArgs::cat) and its allocations
   fk::SceneDev cat = {};
-  void* cat_mem[8] = {};
+  void* cat_mem[9] = {};
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
 };
@@ -204,7 +204,6 @@ int fk_batch_create(fk_ctx* ctx, const fk_batch_job* jobs, uint32_t njobs, int k
     if (rc != FK_OK) return rc;
     fk::BatchJobDev& d = table[i];
     std::memset(&d, 0, sizeof(d));
-    d.s = fk::scene_dev(J.scene);
     d.samples = (const float4*)J.samples->ptr;
     d.coords = (const float4*)J.coords->ptr;
     d.tidx = (const uint32_t*)J.tidx->ptr;
@@ -223,6 +222,10 @@ int fk_batch_create(fk_ctx* ctx, const fk_batch_job* jobs, uint32_t njobs, int k
     d.corner_base = (uint32_t)corners;
     d.root2 = J.scene->wide_count ? (int32_t)recs2 : -1;
     d.root4 = J.scene->wide4_count ? (int32_t)recs4 : -1;
+    d.node_count = J.scene->node_count;
+    d.corner_count = J.scene->corner_count;
+    d.root_is_leaf = J.scene->root_is_leaf;
+    d.filter_ok = J.scene->filter_ok;
     nodes += J.scene->node_count;
     corners += J.scene->corner_count;
     recs2 += J.scene->wide_count;
@@ -292,11 +295,11 @@ int fk_batch_create(fk_ctx* ctx, const fk_batch_job* jobs, uint32_t njobs, int k
   }
   int rc = fk_dev_alloc(ctx, (void**)&b->jobs, sizeof(fk::BatchJobDev) * njobs);
   // the concatenated scene: nodes (lo, hi, jump), corners (positions, normals), triangle records, both layouts,
-  // node boxes side by side
-  const size_t cat_bytes[8] = {16 * (size_t)nodes,   16 * (size_t)nodes,   4 * (size_t)nodes,
+  // node boxes side by side, triangle paths
+  const size_t cat_bytes[9] = {16 * (size_t)nodes,   16 * (size_t)nodes,   4 * (size_t)nodes,
                                16 * (size_t)corners, 16 * (size_t)corners, 64 * (size_t)(corners / 3),
-                               64 * (size_t)recs2,   32 * (size_t)nodes};
-  for (int k = 0; k < 8 && rc == FK_OK; ++k) rc = fk_dev_alloc(ctx, &b->cat_mem[k], std::max<size_t>(cat_bytes[k], 16));
+                               64 * (size_t)recs2,   32 * (size_t)nodes,    8 * (size_t)(corners / 3)};
+  for (int k = 0; k < 9 && rc == FK_OK; ++k) rc = fk_dev_alloc(ctx, &b->cat_mem[k], std::max<size_t>(cat_bytes[k], 16));
   if (rc == FK_OK && recs4) rc = fk_dev_alloc(ctx, (void**)&b->cat.wide4, 128 * (size_t)recs4);
   if (rc == FK_OK) {
     b->cat.node_lo = (const float4*)b->cat_mem[0];
@@ -308,6 +311,7 @@ int fk_batch_create(fk_ctx* ctx, const fk_batch_job* jobs, uint32_t njobs, int k
     b->cat.rec_bary = b->cat.rec + corners / 3;  // the planes of every job's triangles, then their barycentric terms
     b->cat.wide = (const float4*)b->cat_mem[6];
     b->cat.node_box = (const float4*)b->cat_mem[7];
+    b->cat.tri_path = (const uint64_t*)b->cat_mem[8];
     b->cat.node_count = (uint32_t)nodes;
     b->cat.corner_count = (uint32_t)corners;
     b->cat.filter_ok = 1;

@@ -170,7 +170,6 @@ struct SceneDev {
   uint32_t corner_count;
   uint32_t filter_ok;  // scene coordinates small enough for the filtered box test
 };
-SceneDev scene_dev(const fk_scene* s);
 
 // Deepest collapsed (4-wide) tree the 4-wide traversal accepts: it defers at
 // most 3 entries per level within its 64-entry stack.
@@ -230,7 +229,6 @@ void restore_l2(fk_ctx* ctx);
 // One job of a batched hemisphere launch (device-side job table entry).
 static constexpr uint32_t kMaxBatchJobs = 64;
 struct BatchJobDev {
-  SceneDev s;
   const float4* samples;
   const float4* coords;
   const uint32_t* tidx;
@@ -245,11 +243,12 @@ struct BatchJobDev {
   // the job's place in the batch's concatenated scene arrays (BatchArgs::cat)
   uint32_t node_base, corner_base;  // flattened nodes; corners (a multiple of 3)
   int32_t root2, root4;             // root records of the 2-wide and 4-wide layouts
-  uint32_t pad[2];
+  // the job's scene, of which the table keeps no pointer: a scene freed after the batch was made is not read
+  uint32_t node_count, corner_count, root_is_leaf, filter_ok;
 };
 struct BatchArgs {
-  // Every job's scene laid end to end: node, corner and triangle-record
-  // arrays, and both inner layouts, with the jobs' child refs, leaf refs,
+  // Every job's scene laid end to end: node, corner, triangle-record and
+  // triangle-path arrays, and both inner layouts, with the jobs' child refs, leaf refs,
   // triangle ranges and skip pointers offset to the concatenated arrays, so a
   // traversal needs no per-job pointers.
   SceneDev cat;

@@ -1591,7 +1591,7 @@ __global__ void __launch_bounds__(256, FK_BATCH_MIN_BLOCKS) batch_trace_kernel(B
           slo[threadIdx.x] = J.lo;
           hi = J.hi;
           bool done = true;
-          if (id != kMiss && valid_hit(id, J.s.corner_count)) {
+          if (id != kMiss && valid_hit(id, J.corner_count)) {
             f3 o, d, tx, ty;
             texel_frame(s, __ldg(J.coords + g), id + J.corner_base, o, d, tx, ty);
             if (KIND == FK_THICK) d = neg(d);
@@ -1601,25 +1601,25 @@ __global__ void __launch_bounds__(256, FK_BATCH_MIN_BLOCKS) batch_trace_kernel(B
             if (is_ordered(TRAV)) {
               const float4 L = __ldg(s.node_lo + J.node_base), H = __ldg(s.node_hi + J.node_base);
               rp = ray_pre_bounded(o, dir, xyz(L), xyz(H));
-              if (!J.s.filter_ok) rp.exact_only = true;
+              if (!J.filter_ok) rp.exact_only = true;
               float aa;
               if (child_hit<FILTER>(rp, o, dir, xyz(L), xyz(H), hi, aa)) {  // ray_box(o, dir, root) < hi, exactly
                 uint64_t path = 0;
-                if (TRAV == FK_TRAVERSE_ORDERED && J.s.tri_path) path = __ldg(J.s.tri_path + id / 3);
+                if (TRAV == FK_TRAVERSE_ORDERED) path = __ldg(s.tri_path + (id + J.corner_base) / 3);
                 if (TRAV == FK_TRAVERSE_ORDERED && path) {
                   path_start<false, FILTER, 256>(s.wide, rp, myray, J.root2, path, hi, st, stk, tally);
                 } else {
                   st.sp = 0;
-                  st.cur = J.s.root_is_leaf ? kNoRef : (TRAV == FK_TRAVERSE_ORDERED4 ? J.root4 : J.root2);
-                  st.pend = J.s.root_is_leaf ? (int32_t)J.node_base : -1;
+                  st.cur = J.root_is_leaf ? kNoRef : (TRAV == FK_TRAVERSE_ORDERED4 ? J.root4 : J.root2);
+                  st.pend = J.root_is_leaf ? (int32_t)J.node_base : -1;
                 }
                 done = false;
               }
             } else {
               rp = ray_pre(o, dir);
-              if (!J.s.filter_ok) rp.exact_only = true;
+              if (!J.filter_ok) rp.exact_only = true;
               cur = (int32_t)J.node_base;
-              end = J.node_base + J.s.node_count;
+              end = J.node_base + J.node_count;
               done = false;
             }
           } else if (id != kMiss) {
@@ -1674,7 +1674,9 @@ __global__ void __launch_bounds__(256, FK_BATCH_MIN_BLOCKS) batch_trace_kernel(B
 // One job's scene copied into the batch's concatenated arrays: triangle ranges
 // (corner indices in the .w bits) and skip pointers offset by the job's corner
 // and node bases, inner-record refs by its record base, leaf refs
-// -(flat + 1) by its node base.
+// -(flat + 1) by its node base.  Triangle paths are turns from the scene's own
+// root record, so they are copied as they are (0, a start at the root, for a
+// scene without paths).
 __device__ __forceinline__ float cat_ref(float r, uint32_t rec_base, uint32_t node_base) {
   const int32_t v = __float_as_int(r);
   return __int_as_float(v >= 0 ? v + (int32_t)rec_base : v - (int32_t)node_base);
@@ -1744,6 +1746,10 @@ int concat_batch_scene(cudaStream_t st, const fk_scene* s, uint32_t node_base, u
         cudaMemcpyAsync(const_cast<float4*>(cat.rec_bary) + 3 * (size_t)(corner_base / 3), s->tri_rec + nc / 3,
                         48 * (nc / 3), cudaMemcpyDeviceToDevice, st) != cudaSuccess)
       return FK_ERR_CUDA;
+    uint64_t* const paths = const_cast<uint64_t*>(cat.tri_path) + corner_base / 3;
+    if ((s->tri_path ? cudaMemcpyAsync(paths, s->tri_path, 8 * (nc / 3), cudaMemcpyDeviceToDevice, st)
+                     : cudaMemsetAsync(paths, 0, 8 * (nc / 3), st)) != cudaSuccess)
+      return FK_ERR_CUDA;
   }
   return FK_OK;
 }
@@ -1767,7 +1773,7 @@ __global__ void __launch_bounds__(256) batch_reduce_kernel(BatchArgs p) {
   const uint32_t g = t - J.texel_base;
   const float* ts = p.scratch + (J.ray_base + (unsigned long long)g * J.spp - p.r0);
   uint32_t id = __ldg(J.tidx + g);
-  if (id != kMiss && !valid_hit(id, J.s.corner_count)) id = kMiss;
+  if (id != kMiss && !valid_hit(id, J.corner_count)) id = kMiss;
   float* bn = KIND == FK_BN ? J.out0 : (KIND == FK_AO_BN ? J.out1 : nullptr);
   if (id == kMiss) {
     if (KIND == FK_AO || KIND == FK_AO_BN) J.out0[g] = 1.0f;
@@ -1778,7 +1784,7 @@ __global__ void __launch_bounds__(256) batch_reduce_kernel(BatchArgs p) {
     return;
   }
   f3 o, d, tx, ty;
-  if (KIND == FK_BN || KIND == FK_AO_BN) texel_frame(J.s, __ldg(J.coords + g), id, o, d, tx, ty);
+  if (KIND == FK_BN || KIND == FK_AO_BN) texel_frame(p.cat, __ldg(J.coords + g), id + J.corner_base, o, d, tx, ty);
   const float4* row = J.samples + (size_t)(g % J.perms) * J.spp;
   uint32_t occ = 0, anyhit = 0;
   float acc = 0.0f;
@@ -1814,8 +1820,6 @@ __global__ void __launch_bounds__(256) batch_reduce_kernel(BatchArgs p) {
     J.hits0[g] = KIND == FK_AO ? occ : anyhit;
   }
 }
-
-SceneDev scene_dev(const fk_scene* s) { return dev_of(s); }
 
 template <int KIND, int TRAV, bool FILTER>
 static cudaError_t batch_launch(const BatchArgs& a, cudaStream_t stream, int sm_count, bool reduce) {

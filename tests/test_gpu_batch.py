@@ -145,3 +145,30 @@ def test_batch_with_a_job_run_alone(ctx, setup):
     ctx.sync()
     ctx.check()
     check(jobs, outs, kind, want)
+
+
+def test_batch_reads_no_freed_scene(ctx, setup):
+    """The jobs that share launches read the batch's own copy of their scenes:
+    with the scenes freed and their memory written over, runs and replays still
+    give each job its result."""
+    meshes = [cases.sphere().hm, cases.plane().hm]
+    scenes = [api.Scene.build(ctx, m) for m in meshes]
+    scenes[1].set_tree(api.TREE_REFERENCE)
+    jobs = [dict(setup[i], scene=s) for i, s in enumerate(scenes)]
+    kind = api.AO_BN
+    want = [alone(ctx, j, kind, api.TRAVERSE_ORDERED) for j in jobs]
+    b, outs = make_batch(ctx, jobs, kind)
+    b.capture(api.TRAVERSE_ORDERED)
+    sizes = [s.info()["device_bytes"] for s in scenes]
+    for s in scenes:
+        s.free()
+    over = [ctx.upload(np.full(n // 2, 0xA5, np.uint8)) for n in sizes for _ in range(2)]
+    for again in (lambda: b.run(api.TRAVERSE_ORDERED), b.replay):
+        for o in outs:
+            for buf in o:
+                buf.upload(np.zeros(buf.nbytes, np.uint8))
+        again()
+        ctx.sync()
+        check(jobs, outs, kind, want)
+    ctx.check()
+    del over
