@@ -785,6 +785,7 @@ class Batch:
         self.ctx = ctx
         arr = (L.BatchJob * len(jobs))()
         hv = lambda b: b.handle if b is not None else None
+        self._keep = [dict(j) for j in jobs]  # scenes and buffers live as long as the batch that reads them
         for i, j in enumerate(jobs):
             arr[i] = L.BatchJob(j["scene"].handle, j["coords"].handle, j["tidx"].handle, j["texel_count"],
                                 L.SampleParams(j["spp"], j.get("perms", PERMS), j["min_distance"], j["max_distance"]),
@@ -819,6 +820,7 @@ class Batch:
         if self.handle and self.ctx.handle:
             self.ctx.lib.fk_batch_free(self.handle)
         self.handle = None
+        self._keep = None
 
     def __del__(self):
         try:

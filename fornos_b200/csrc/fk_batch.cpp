@@ -37,6 +37,7 @@ constexpr unsigned long long kSoloRays = FK_BATCH_SOLO_RAYS;
 // A job run alone (fk_batch's `solo`): its scene and its launch.
 struct Solo {
   const fk_scene* scene;
+  uint64_t serial;  // fk_scene::serial
   fk::HemiLaunch h;
 };
 
@@ -69,6 +70,14 @@ struct fk_batch {
 };
 
 static bool fits(const fk_buf* b, uint64_t bytes) { return b && b->bytes >= bytes; }
+
+// A job that runs alone reads its scene at every run: refused once the scene is freed.
+static int solo_scenes_alive(const fk_batch* b, const char* who) {
+  for (const Solo& j : b->solo)
+    if (!b->ctx->scenes.count(const_cast<fk_scene*>(j.scene)) || j.scene->serial != j.serial)
+      return fk_fail(b->ctx, FK_ERR_INVALID, std::string(who) + ": the scene of a job that runs alone was freed");
+  return FK_OK;
+}
 
 static int batch_run_chunks(fk_batch* b, int trav, bool filter, const fk_tuning& tun) {
   fk_ctx* ctx = b->ctx;
@@ -255,6 +264,7 @@ int fk_batch_create(fk_ctx* ctx, const fk_batch_job* jobs, uint32_t njobs, int k
       const fk_batch_job& J = jobs[i];
       Solo so;
       so.scene = J.scene;
+      so.serial = J.scene->serial;
       so.h.kind = kind;
       so.h.spp = J.params.sample_count;
       so.h.perms = J.params.perm_count;
@@ -439,6 +449,8 @@ int fk_batch_run(fk_batch* b, int traverse) {
     return fk_fail(b->ctx, FK_ERR_INVALID, "fk_batch_run: unknown traversal");
   if (trav == FK_TRAVERSE_ORDERED4 && !b->ordered4_ok)
     return fk_fail(b->ctx, FK_ERR_INVALID, "fk_batch_run: a job's tree is too deep for the 4-wide traversal");
+  const int rc = solo_scenes_alive(b, "fk_batch_run");
+  if (rc != FK_OK) return rc;
   return batch_run_chunks(b, trav, filter, b->tuning);
 }
 
@@ -467,6 +479,8 @@ int fk_batch_capture(fk_batch* b, int traverse) {
 int fk_batch_replay(fk_batch* b) {
   if (!b) return FK_ERR_INVALID;
   if (!b->exec) return fk_fail(b->ctx, FK_ERR_STATE, "fk_batch_replay: nothing captured");
+  const int rc = solo_scenes_alive(b, "fk_batch_replay");
+  if (rc != FK_OK) return rc;
   FK_CUDA(b->ctx, cudaGraphLaunch(b->exec, b->ctx->stream));
   b->ctx->launches += 2 * b->chunks.size() + b->solo_launches;
   return FK_OK;

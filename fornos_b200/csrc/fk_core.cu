@@ -349,6 +349,7 @@ static int scene_create(fk_ctx* ctx, const fk_bvh_node* nodes, uint32_t nn, cons
     return FK_ERR_NOMEM;
   }
   s->ctx = ctx;
+  s->serial = ++ctx->scenes_made;
   s->node_count = nn;
   s->corner_count = nc;
   s->depth = maxd;

@@ -45,6 +45,7 @@ struct fk_ctx {
   size_t l2_prev_limit = 0;
   std::set<fk_buf*> bufs;
   std::set<fk_scene*> scenes;
+  uint64_t scenes_made = 0;
   std::set<fk_texel_map*> maps;
 };
 
@@ -56,6 +57,7 @@ struct fk_buf {
 
 // High-poly mesh + BVH on the device.
 struct fk_scene {
+  uint64_t serial = 0;  // nth scene of its context: told apart from a later one at the same address
   fk_ctx* ctx = nullptr;
   uint32_t node_count = 0, corner_count = 0, depth = 0, leaf_count = 0;
   // Reference layout, one entry per flattened node (skip-pointer walk):

@@ -432,7 +432,11 @@ int fk_solver_free(fk_solver* s);
  * every lane maps its ray back to its job, so small jobs keep the whole GPU
  * busy together.  A job of 2^21 rays or more runs alone through the
  * single-job path within the same run (and the same graph), on the batch's
- * scratch.  Results are those fk_hemisphere gives per job. */
+ * scratch.  Results are those fk_hemisphere gives per job.
+ * A batch copies the scenes of the jobs that share launches when it is made;
+ * the scene of a job that runs alone must outlive the batch's runs (a run or a
+ * replay after it was freed is refused with FK_ERR_INVALID), and so must every
+ * job's buffers. */
 typedef struct fk_batch fk_batch;
 typedef struct fk_batch_job {
   const fk_scene* scene;

@@ -172,3 +172,31 @@ def test_batch_reads_no_freed_scene(ctx, setup):
         check(jobs, outs, kind, want)
     ctx.check()
     del over
+
+
+def test_batch_refuses_a_freed_scene_of_a_job_run_alone(ctx, setup):
+    """A job of 2^21 rays reads its scene at every run: a run, a capture and a
+    replay after the scene was freed are refused, also when another scene takes
+    its place, and a batch keeps the scenes it was given alive."""
+    mesh = cases.sphere().hm
+    n = setup[0]["texel_count"]
+    spp = (1 << 21) // n + 1
+    table = ctx.upload(api.samples_cosine(spp, 1, 5))
+
+    def made():
+        return make_batch(ctx, [dict(setup[0], scene=api.Scene.build(ctx, mesh), spp=spp, perms=1, samples=table)], api.AO)
+
+    b, outs = made()  # the scene's only reference is the batch's
+    b.capture(api.TRAVERSE_ORDERED)
+    b.run(api.TRAVERSE_ORDERED)
+    b.replay()
+    ctx.sync()
+    scene = b._keep[0]["scene"]
+    scene.free()
+    others = [api.Scene.build(ctx, mesh) for _ in range(8)]
+    for call in (lambda: b.run(api.TRAVERSE_ORDERED), b.replay, lambda: b.capture(api.TRAVERSE_ORDERED)):
+        with pytest.raises(api.FornosError) as e:
+            call()
+        assert e.value.code == -1 and "was freed" in str(e.value)
+    ctx.check()
+    del others
