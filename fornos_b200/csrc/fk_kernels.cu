@@ -1422,7 +1422,7 @@ static int run_hemi_dynamic(fk_ctx* ctx, const HemiArgs& a, uint32_t refill, boo
   trace_shape(ctx->tuning, a, TRAV, filter, x.odepth, x.top_count > 0, &block, &stack);
   auto trace = pick_trace<KIND, TRAV>(a.tally != nullptr, filter, block, stack, x.top_count > 0);
   const size_t smem = 64 * (size_t)x.top_count;
-  if (smem > 48 * 1024) {
+  if (smem) {  // static and staged shared memory together pass the default 48 KB from 609 records on
     cudaError_t e = cudaFuncSetAttribute(trace, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fk_cuda_fail(ctx, e, "cudaFuncSetAttribute");
   }

@@ -52,3 +52,28 @@ def test_path_start_equals_skip_walk(quads, max_tris, tree):
     assert got[2][1].max() > 0 or nt <= 8
     for out, hits in got:
         assert np.array_equal(out, got[2][0]) and np.array_equal(hits, got[2][1])
+
+
+@pytest.mark.parametrize("top", [1, 64, 608, 609, 640, 641, 768, 1024])
+def test_staged_records_of_every_size(top):
+    """Staged top records take the trace kernel's shared memory past the default
+    limit within their allowed range; every size runs and gives the same counts."""
+    ctx = api.Context(0)
+    mesh = api.Mesh(flat(64, 3))
+    mesh.compute_vertex_normals()
+    scene = api.Scene.build(ctx, mesh, 1)
+    n, nt = 500, 2 * 64 * 64
+    rng = np.random.default_rng(6)
+    coords = np.zeros((n, 4), np.float32)
+    coords[:, 1:] = rng.dirichlet((1, 1, 1), n)
+    cb, tb = ctx.upload(coords), ctx.upload((3 * rng.integers(0, nt, n)).astype(np.uint32))
+    table = ctx.upload(api.samples_cosine(SPP, 16, 3))
+    got = []
+    for knobs, traverse in ((dict(top_records=top), api.TRAVERSE_ORDERED), (dict(top_records=0), api.TRAVERSE_SKIP)):
+        ctx.set_tuning(**knobs)
+        hits = ctx.buffer(4 * n)
+        api.hemisphere(ctx, scene, cb, tb, api.AO, SPP, LO, HI, table, ctx.buffer(4 * n), None, hits, None, 0, n, 16,
+                       traverse)
+        got.append(hits.download(np.uint32, n))
+    ctx.check()
+    assert got[0].max() > 0 and np.array_equal(*got)
