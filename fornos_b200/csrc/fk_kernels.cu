@@ -1018,9 +1018,21 @@ __device__ __forceinline__ bool skip_step(const SceneDev& s, const RayPre& rp, c
 
 // Inner visits a lane makes per iteration of the trace loop before the warp
 // decides its next phase again (the phase ballots and the refill check are
-// paid once per kInnerVisits visits).  4 / 6 / 8: 21.50 / 21.29 / 21.25 ms (AO +
-// BN, 500 x 500 texels, 256 spp, 2.1M triangles).
-constexpr int kInnerVisits = 8;
+// paid once per inner_visits visits).  2-wide, 4 / 6 / 8: 21.50 / 21.29 / 21.25
+// ms (AO + BN, 500 x 500 texels, 256 spp, 2.1M triangles).  The 4-wide visit is
+// three times as long: 4 of them, and its loop is not unrolled, which spilled
+// (AO of 200 x 200 texels at 64 spp on 500k triangles: 8 visits unrolled 1.57 ms,
+// with divided box tests 4.66; 4 not unrolled 1.25 and 1.72).  Divided box tests
+// keep their loop rolled for the same reason (2-wide 1.88 against 1.39 ms), the
+// filtered 2-wide visit gains 2 % from the unrolling.
+template <int TRAV>
+__host__ __device__ constexpr int inner_visits() {
+  return TRAV == FK_TRAVERSE_ORDERED4 ? 4 : 8;
+}
+template <int TRAV, bool FILTER>
+__host__ __device__ constexpr int visits_unrolled() {
+  return TRAV == FK_TRAVERSE_ORDERED && FILTER ? inner_visits<TRAV>() : 1;
+}
 
 // BLOCK: threads per block; STACK: deferred entries per lane (the ordered
 // traversals accept trees of depth below STACK, the 4-wide one of depth up
@@ -1140,7 +1152,8 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 512 ? 2 : 1280 / BLOCK) hemi_t
           if (visited) fin = settled<STOP>(best, p.hi);
           next_ref(st, stk);
         } else {
-          for (int v = 0; v < kInnerVisits && st.cur >= 0 && (st.pend < 0 || p.speculate); ++v) {
+#pragma unroll (visits_unrolled<TRAV, FILTER>())
+          for (int v = 0; v < inner_visits<TRAV>() && st.cur >= 0 && (st.pend < 0 || p.speculate); ++v) {
             if (!visit_inner<TRAV, COUNT, FILTER, BLOCK, STACK, TOP>(p.s, rp, myray, fminf(best, p.hi), st, stk,
                                                                       p.status, tally, top_smem, top_base)) {
               fin = true;
@@ -1646,7 +1659,8 @@ __global__ void __launch_bounds__(256, FK_BATCH_MIN_BLOCKS) batch_trace_kernel(B
           if (visited) fin = settled<STOP>(best, hi);
           next_ref(st, stk);
         } else {
-          for (int v = 0; v < kInnerVisits && st.cur >= 0 && (st.pend < 0 || p.speculate); ++v) {
+#pragma unroll (visits_unrolled<TRAV, FILTER>())
+          for (int v = 0; v < inner_visits<TRAV>() && st.cur >= 0 && (st.pend < 0 || p.speculate); ++v) {
             if (!visit_inner<TRAV, false, FILTER, 256>(s, rp, myray, fminf(best, hi), st, stk, p.status, tally)) {
               fin = true;
               break;
