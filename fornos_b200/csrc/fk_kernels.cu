@@ -968,16 +968,24 @@ __device__ __forceinline__ bool leaf_phase_warp(const SceneDev& s, const RayPre&
 // 1024 texels at 256 spp on that heightfield from 120.0 to 105.4 ms (87.0 with the
 // leaf phase and lane state below) and AO of 512 x 512 texels at 64 spp on the
 // 261k-triangle sphere from 5.59 to 4.74 ms (3.94).
-template <bool COUNT, bool FILTER, int S>
+// TOP: the way down starts in the staged records, whose child refs name staged
+// records, so the siblings deferred there are read from shared memory as well.
+template <bool COUNT, bool FILTER, int S, bool TOP = false>
 __device__ __forceinline__ void path_start(const float4* __restrict__ wide, const RayPre& rp, const float* ray,
                                            int32_t root, uint64_t path, float hi, OState& st, int32_t* stk,
-                                           Tally& tally) {
+                                           Tally& tally, const float4* top = nullptr, uint32_t top_base = 0) {
   int32_t ref = root;
   int sp = 0;
   while (path > 1) {
-    const float4* w = wide + 4 * (size_t)ref;
     const bool second = path & 1;
-    const float4 xy = __ldg(w + (second ? 0 : 1)), z = __ldg(w + 2), w3 = __ldg(w + 3);
+    float4 xy, z, w3;
+    if (TOP && (uint32_t)ref >= top_base) {
+      const float4* w = top + 4 * ((uint32_t)ref - top_base);
+      xy = w[second ? 0 : 1], z = w[2], w3 = w[3];
+    } else {
+      const float4* w = wide + 4 * (size_t)ref;
+      xy = __ldg(w + (second ? 0 : 1)), z = __ldg(w + 2), w3 = __ldg(w + 3);
+    }
     float entry;
     if (COUNT) tally.box++;
     const bool h = child_maybe<FILTER, S>(rp, ray, mk3(xy.x, xy.z, second ? z.x : z.z),
@@ -1104,9 +1112,10 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 512 ? 2 : 1280 / BLOCK) hemi_t
               if (COUNT) tally.box++;
               if (child_hit<FILTER>(rp, o, dir, xyz(L), xyz(H), p.hi, a)) {  // ray_box(o, dir, root) < hi, exactly
                 uint64_t path = 0;
-                if (TRAV == FK_TRAVERSE_ORDERED && !TOP && p.s.tri_path) path = __ldg(p.s.tri_path + id / 3);
-                if (TRAV == FK_TRAVERSE_ORDERED && !TOP && path) {
-                  path_start<COUNT, FILTER, BLOCK>(p.s.wide, rp, myray, 0, path, p.hi, st, stk, tally);
+                if (TRAV == FK_TRAVERSE_ORDERED && p.s.tri_path) path = __ldg(p.s.tri_path + id / 3);
+                if (TRAV == FK_TRAVERSE_ORDERED && path) {
+                  path_start<COUNT, FILTER, BLOCK, TOP>(p.s.wide, rp, myray, TOP ? (int32_t)top_base : 0, path, p.hi,
+                                                        st, stk, tally, top_smem, top_base);
                 } else {
                   st.sp = 0;
                   st.cur = p.s.root_is_leaf ? kNoRef : (TOP ? (int32_t)top_base : 0);
