@@ -2262,7 +2262,7 @@ __device__ bool map_line(const SceneDev& s, f3 o, f3 d, float max_d, float& t, u
         const float4 cl = __ldg(s.chain_box + 2 * (size_t)(-(cur + 1))), ch = __ldg(s.chain_box + 2 * (size_t)(-(cur + 1)) + 1);
         const bool visited = ray_box(o, wk ? neg(d) : d, xyz(cl), xyz(ch)) <= at;
         sure = at < best ? visited : sure && visited;
-        best = at;
+        best = wk ? -th : th;  // the walk's own distance: -0 stays -0
         corner = k;
         walk = wk;
         w = q;
