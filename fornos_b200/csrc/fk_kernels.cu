@@ -2085,8 +2085,9 @@ __device__ float walk_twoside(const SceneDev& s, f3 o, f3 d, float mint, uint32_
 // the walks' own box test on the box that the leaf and its ancestors have in
 // common (chain_box; the flattened boxes are rounded from centre and half size
 // and do not nest exactly; the test is monotone, so each of them is entered no
-// later).  A texel for which it fails (a hit that rounds to before its leaf's
-// box, a ray in a box face) takes the walks.
+// later, as long as they have a point in common).  A texel for which it fails (a
+// hit that rounds to before its leaf's box, a ray in a box face, a leaf outside
+// an ancestor's rounded box) takes the walks.
 //
 // It finds every hit up to t*: a hit lies within map_pad + 128 u M' of its
 // triangle's box (u = 2^-24, M' the largest coordinate of scene and origin).
@@ -2140,6 +2141,9 @@ __global__ void map_pad_kernel(const float4* __restrict__ lo, const float4* __re
         }
       }
       if (steps > kMaxChain) p = inf;  // an uploaded tree of extreme depth: the walks
+      // A flat leaf at an ancestor's rounded face can lie an ulp outside it.  Nothing is then in both boxes, and the
+      // box test would swap the faces and report an entry before the ancestor's: a box that no ray enters instead.
+      if (cl.x > ch.x || cl.y > ch.y || cl.z > ch.z) cl.x = ch.x = cl.y = ch.y = cl.z = ch.z = __int_as_float(0x7fffffff);
       chain[2 * (size_t)i] = make_float4(cl.x, cl.y, cl.z, 0.0f);
       chain[2 * (size_t)i + 1] = make_float4(ch.x, ch.y, ch.z, 0.0f);
     }

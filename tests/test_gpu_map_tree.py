@@ -90,3 +90,39 @@ def test_tree_route_equals_walks(name, cull):
         assert np.array_equal(bits(c1[:, 1:]), bits(c8[:, 1:]))
         assert hit.sum() > 100 or name in ("two", "nine", "flat")
     ctx.check()
+
+
+@pytest.mark.parametrize("cull", [True, False])
+@pytest.mark.parametrize("seed", range(4))
+def test_flat_face_outside_its_ancestors_rounded_box(cull, seed):
+    """The root's box, rounded from centre and half size, ends an ulp below the
+    mesh's flat top: a walk enters it only behind the hit, so a maximum distance
+    in between makes the texel a miss."""
+    rng = np.random.default_rng(seed)
+    f = np.float32
+    while True:
+        lo, hi = f(-rng.uniform(0.1, 3.0)), f(rng.uniform(0.5, 1.0))
+        top = (lo + hi) * f(0.5) + (hi - lo) * f(0.5)
+        if top < hi:
+            break
+    quads, n = 8, 64
+    m = W.grid_plane(quads, heights=np.full((quads + 1) ** 2, hi))
+    nv = len(m.positions)
+    pos = np.concatenate([m.positions, [[0, 0, lo], [1, 0, lo], [0, 1, lo]]]).astype(f)
+    verts = np.stack([np.arange(nv + 3), np.zeros(nv + 3), np.zeros(nv + 3)], -1)
+    mesh = api.Mesh(W.MeshArrays(pos, m.texcoords[:1], [[0, 0, 1]], verts,
+                                 np.concatenate([m.triangles, [[nv, nv + 1, nv + 2]]])))
+    ctx = api.Context(0)
+    scene = api.Scene.build(ctx, mesh)
+    o = np.zeros((n, 3), f)
+    o[:, :2] = rng.uniform(0.05, 0.95, (n, 2))
+    o[:, 2] = f(1.25) * hi  # both differences below are exact
+    d = np.tile([[0, 0, 1]], (n, 1)).astype(f)
+    hit, entry = o[0, 2] - hi, o[0, 2] - top
+    assert entry > hit
+    for max_d, found in ((entry, False), (np.nextafter(entry, f(9)), True), (api.FLT_MAX, True)):
+        far = max_d if max_d == api.FLT_MAX else max_d / 8
+        c1, t1 = mapped(ctx, scene, o, d, cull, float(max_d))
+        c8, t8 = mapped(ctx, scene, o, 8 * d, cull, float(far))
+        assert np.array_equal(t1 != api.MISS, np.full(n, found)) and np.array_equal(t1, t8)
+        assert np.array_equal(bits(c1[:, 1:]), bits(c8[:, 1:])) and (not found or np.all(c1[:, 0] == hit))
