@@ -199,6 +199,8 @@ _SIGS = {
                                          c_u32, c_int, ctypes.POINTER(c_u64)]),
     "fk_diag_traversal_profile": (c_int, [c_vp, c_vp, c_vp, c_vp, c_int, ctypes.POINTER(SampleParams), c_vp, c_u32,
                                           c_u32, c_int, ctypes.POINTER(c_u64)]),
+    "fk_diag_meshmap_routes": (c_int, [c_vp, c_vp, c_vp, c_int, ctypes.c_float, ctypes.POINTER(c_u32),
+                                       ctypes.POINTER(ctypes.c_float)]),
     "fk_bvh_build_flat": (c_int, [c_vp, c_vp, c_u32, c_u32, c_vp, c_u32, ctypes.POINTER(c_u32), f32p, f32p]),
     "fk_scene_build": (c_int, [c_vp, c_vp, c_u32, c_u32, ctypes.POINTER(c_vp)]),
     "fk_export_image": (c_int, [c_vp, c_vp, c_vp, ctypes.POINTER(ExportParams), c_vp, f32p]),

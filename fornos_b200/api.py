@@ -704,6 +704,15 @@ def traversal_profile(ctx, scene, coords, tidx, kind, spp, min_d, max_d, samples
     return dict(zip(PROFILE_KEYS, (int(v) for v in out)))
 
 
+def meshmap_routes(ctx, scene, tmap, cull_backfaces, max_dist=FLT_MAX):
+    """Texels of the map that the mapping's tree route answers, and the leaves its bound makes a ray meet
+    (fk_diag_meshmap_routes)."""
+    n, reach = L.c_u32(), ctypes.c_float()
+    _check(ctx.lib.fk_diag_meshmap_routes(ctx.handle, scene.handle, tmap.handle, int(cull_backfaces), max_dist,
+                                          ctypes.byref(n), ctypes.byref(reach)), ctx, "mapping routes")
+    return n.value, reach.value
+
+
 def _sampler(cfg):
     if not cfg:
         return L.BakeSampler(0, 0, 0.0, 0.0, 0, 0)

@@ -3,6 +3,7 @@
 // (Src/meshmapping.cpp:128-218) and the six solvers (Src/solver_*.cpp), with
 // the reference's init / runStep / getResults / progress contract.
 #include <cfloat>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
@@ -29,6 +30,30 @@ int fk_meshmap(fk_ctx* ctx, const fk_scene* s, const fk_texel_map* m, int cull, 
   if (!fits(coords, 16 * end) || !fits(tidx, 4 * end))
     return fk_fail(ctx, FK_ERR_INVALID, "fk_meshmap: output buffers too small");
   return fk::launch_meshmap(ctx, s, m, cull, max_dist, offset, count, (float4*)coords->ptr, (uint32_t*)tidx->ptr);
+}
+
+int fk_diag_meshmap_routes(fk_ctx* ctx, const fk_scene* s, const fk_texel_map* m, int cull, float max_dist,
+                           uint32_t* tree_texels, float* reach) {
+  if (!ctx || !s || !m || !tree_texels) return fk_fail(ctx, FK_ERR_INVALID, "fk_diag_meshmap_routes: null argument");
+  if (!(max_dist > 0.0f)) return fk_fail(ctx, FK_ERR_INVALID, "fk_diag_meshmap_routes: max_dist must be positive");
+  *tree_texels = 0;
+  if (reach) *reach = s->map_pad <= FLT_MAX ? s->map_reach : HUGE_VALF;
+  if (!s->map_tree || !m->count) return FK_OK;
+  void *coords = nullptr, *tidx = nullptr, *count = nullptr;
+  int rc = fk_dev_alloc(ctx, &coords, 16 * (size_t)m->count);
+  if (rc == FK_OK) rc = fk_dev_alloc(ctx, &tidx, 4 * (size_t)m->count);
+  if (rc == FK_OK) rc = fk_dev_alloc(ctx, &count, 4);
+  cudaError_t e = cudaSuccess;
+  if (rc == FK_OK) e = cudaMemsetAsync(count, 0, 4, ctx->stream);
+  if (rc == FK_OK && e == cudaSuccess)
+    rc = fk::launch_meshmap(ctx, s, m, cull, max_dist, 0, m->count, (float4*)coords, (uint32_t*)tidx, (uint32_t*)count);
+  if (rc == FK_OK && e == cudaSuccess)
+    e = cudaMemcpyAsync(tree_texels, count, 4, cudaMemcpyDeviceToHost, ctx->stream);
+  if (rc == FK_OK && e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  fk_dev_free(ctx, coords);
+  fk_dev_free(ctx, tidx);
+  fk_dev_free(ctx, count);
+  return rc == FK_OK && e != cudaSuccess ? fk_cuda_fail(ctx, e, "fk_diag_meshmap_routes") : rc;
 }
 
 int fk_hemisphere(fk_ctx* ctx, const fk_scene* s, const fk_buf* coords, const fk_buf* tidx, int kind,

@@ -455,14 +455,9 @@ static int scene_create(fk_ctx* ctx, const fk_bvh_node* nodes, uint32_t nn, cons
     if (e != cudaSuccess) rc = fk_cuda_fail(ctx, e, "pair_boxes_kernel");
     else ++ctx->launches;
   }
-  if (rc == FK_OK) rc = fk_dev_alloc(ctx, (void**)&s->map_pad, sizeof(float));
-  if (rc == FK_OK) {
-    rc = fk_dev_alloc(ctx, (void**)&s->chain_box, 2 * sizeof(float4) * (size_t)nn);
-    s->bytes += 2 * sizeof(float4) * (size_t)nn;
-  }
-  if (rc == FK_OK) rc = fk::launch_map_pad(ctx, s);
   if (rc == FK_OK)
     rc = fk::ensure_tri_path(ctx, s, s->tree_wide[FK_TREE_SAH] ? FK_TREE_SAH : FK_TREE_REFERENCE);
+  if (rc == FK_OK) rc = fk::launch_map_bound(ctx, s);
   if (rc == FK_OK) {
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) rc = fk_cuda_fail(ctx, e, "scene upload sync");
@@ -570,7 +565,7 @@ int fk_scene_free(fk_ctx* ctx, fk_scene* s) {
   cudaStreamSynchronize(ctx->stream);
   void* ps[] = {s->node_lo,         s->node_hi,         s->node_jump, s->pos4,    s->nrm4,  s->tree_wide[0],
                 s->tree_wide[1],   s->tree_wide4[0],   s->tree_wide4[1], s->tri_rec, s->top, s->node_box,
-                s->tree_path[0],   s->tree_path[1],    s->map_pad,       s->chain_box};
+                s->tree_path[0],   s->tree_path[1],    s->chain_box};
   for (void* p : ps) fk_dev_free(ctx, p);
   ctx->scenes.erase(s);
   delete s;

@@ -82,7 +82,9 @@ struct fk_scene {
   float4* wide4 = nullptr;
   uint32_t wide4_count = 0, depth4 = 0;
   float4* tri_rec = nullptr;
-  float* map_pad = nullptr;      // SceneDev::map_pad
+  float map_pad = 0.0f;          // SceneDev::map_pad
+  float map_reach = 0.0f;        // leaves that pad makes a mapping ray meet round its own (launch_map_bound)
+  bool map_tree = false;         // mapping walks the surface-area tree
   float4* chain_box = nullptr;   // SceneDev::chain_box
   // Root-to-leaf path of each triangle's leaf in the 2-wide tree (SceneDev::tri_path): the active tree's, and
   // both trees' once built.  Null for a single leaf or a tree deeper than kMaxOrderedDepth.
@@ -158,10 +160,10 @@ struct SceneDev {
   // read only for hits inside the distance range.
   const float4* __restrict__ rec;
   const float4* __restrict__ rec_bary;
-  // One value: how far outside its own box a triangle's mapping hit can lie (map_pad_kernel), infinite where the
-  // tree walk of the mapping has no such bound and the skip-pointer walk runs instead.
-  const float* __restrict__ map_pad;
-  // Per leaf i of the flattened nodes, the box that it and all nodes above it have in common (lo, hi at 2 i, 2 i + 1).
+  // How far outside its own box a triangle's mapping hit can lie (map_pad_kernel).
+  float map_pad;
+  // Per leaf i of the flattened nodes, the box that it and all nodes above it have in common (lo, hi at 2 i, 2 i + 1);
+  // null where the mapping takes the skip-pointer walks.
   const float4* __restrict__ chain_box;
   const float4* __restrict__ sah;  // the surface-area tree's records, whichever tree is active; null: none
   // Per triangle, the way from the 2-wide tree's root record to the leaf that holds it: bit k is the child taken
@@ -272,8 +274,9 @@ cudaError_t launch_batch(const BatchArgs& a, int kind, int trav, bool filter, cu
 // (nodes, corners, 2-wide and 4-wide records), offsetting its refs.
 int concat_batch_scene(cudaStream_t st, const fk_scene* s, uint32_t node_base, uint32_t corner_base, uint32_t rec2,
                        uint32_t rec4, const SceneDev& cat);
+// by_tree: device counter of the texels that the tree route answers, or null.
 int launch_meshmap(fk_ctx* ctx, const fk_scene* s, const fk_texel_map* m, int cull, float max_d, uint32_t offset,
-                   uint32_t count, float4* coords, uint32_t* tidx);
+                   uint32_t count, float4* coords, uint32_t* tidx, uint32_t* by_tree = nullptr);
 struct HemiLaunch {
   int kind;
   uint32_t spp, perms;
@@ -310,8 +313,9 @@ int launch_gather(fk_ctx* ctx, const fk_scene* s, int kind, const float4* coords
                   uint32_t offset, uint32_t count, float* out);
 int launch_tangent_space(fk_ctx* ctx, const fk_texel_map* m, uint32_t offset, uint32_t count, float* io3);
 int launch_tri_records(fk_ctx* ctx, fk_scene* s);
-// Fills fk_scene::map_pad and chain_box from the scene's nodes, corners and triangle records.
-int launch_map_pad(fk_ctx* ctx, fk_scene* s);
+// Decides the mapping's route (fk_scene::map_tree) and fills map_pad, map_reach and chain_box from the scene's nodes,
+// corners, triangle records and surface-area tree.
+int launch_map_bound(fk_ctx* ctx, fk_scene* s);
 // fk_scene::tree_path[tree], built on first use (no-op where the tree has none).
 int ensure_tri_path(fk_ctx* ctx, fk_scene* s, int tree);
 // Fills box[2 i], box[2 i + 1] = lo[i], hi[i] for i < n on `stream`.

@@ -2105,8 +2105,9 @@ __device__ float walk_twoside(const SceneDev& s, f3 o, f3 d, float mint, uint32_
 // map_pad_kernel gives an infinite bound where this does not hold: s below
 // 2^-24, edges outside [2^-25, 2^25], a triangle outside its leaf's box or the
 // root's coordinates (an uploaded scene); a triangle whose normal is NaN is
-// never hit.  Directions far from unit length and
-// coordinates from 2^24 up take the walks too.
+// never hit.  Scenes without a bound, or with one that makes the traversal meet
+// too many leaves (kMaxMapReach), take the walks altogether; directions far from
+// unit length and origins from 2^24 up take them too.
 //
 // Bound by the latency of the record and triangle loads.  The walks divide six
 // times a node and visit hundreds of the reference tree's nodes a ray.
@@ -2168,13 +2169,75 @@ __global__ void map_pad_kernel(const float4* __restrict__ lo, const float4* __re
   if ((threadIdx.x & 31) == 0 && p > 0.0f) atomicMax(pad, __float_as_uint(p));
 }
 
-int launch_map_pad(fk_ctx* ctx, fk_scene* s) {
-  if (!s->tree_wide[FK_TREE_SAH]) return FK_OK;  // nothing reads it (launch_meshmap)
-  const cudaError_t e = cudaMemsetAsync(s->map_pad, 0, sizeof(float), ctx->stream);
-  if (e != cudaSuccess) return fk_cuda_fail(ctx, e, "mapping bound");
-  map_pad_kernel<<<(s->node_count + 255) / 256, 256, 0, ctx->stream>>>(s->node_lo, s->node_hi, s->node_jump, s->pos4,
-                                                                       s->tri_rec, s->node_count, (uint32_t*)s->map_pad, s->chain_box);
-  return fk_after_launch(ctx, "map_pad_kernel");
+// Sum over the leaves of how many leaves of the same size a mapping ray meets
+// because of the pad: (1 + 2 p / e1)(1 + 2 p / e2) for a surface's leaf of sides
+// e1 >= e2, each factor at most 64, in sixteenths (whole numbers: any order of
+// the sums gives the same).
+__global__ void map_reach_kernel(const float4* __restrict__ lo, const float4* __restrict__ hi, uint32_t nodes,
+                                 const float* __restrict__ bound, unsigned long long* __restrict__ sum) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t v = 0;
+  if (i < nodes) {
+    const float4 L = lo[i], H = hi[i], RL = lo[0], RH = hi[0];
+    if (as_u32(L.w) < as_u32(H.w)) {
+      const float M = fmaxf(fmaxf(fmaxf(fabsf(RL.x), fabsf(RH.x)), fmaxf(fabsf(RL.y), fabsf(RH.y))),
+                            fmaxf(fabsf(RL.z), fabsf(RH.z)));
+      const float p2 = 2.0f * (*bound + M * 7.62939453e-06f);  // the pad of a ray from inside the root box
+      const float x = H.x - L.x, y = H.y - L.y, z = H.z - L.z;
+      const float e1 = fmaxf(fmaxf(x, y), z), e2 = fmaxf(fminf(x, y), fminf(fmaxf(x, y), z));
+      v = (uint32_t)(16.0f * fminf(1.0f + p2 / e1, 64.0f) * fminf(1.0f + p2 / e2, 64.0f));
+    }
+  }
+  v = __reduce_add_sync(0xFFFFFFFFu, v);
+  if ((threadIdx.x & 31) == 0 && v) atomicAdd(sum, (unsigned long long)v);
+}
+
+// The tree route's time grows with the leaves that the pad adds, the walks' does
+// not.  1024 x 1024 texels on a 2M-triangle heightfield with one triangle whose
+// edges meet at a thin angle, mean leaves met / tree / walks: 1.2 / 0.38 / 1.18
+// ms (0.1 rad), 4.7 / 0.83 / 1.18 (0.003), 17.9 / 2.26 / 1.18 (0.001), 166 / 17.0
+// / 1.18 (0.00026).  The two meet at about 8.
+constexpr float kMaxMapReach = 6.0f;
+
+int launch_map_bound(fk_ctx* ctx, fk_scene* s) {
+  // a rebuilt tree (kept only where it fits the stack; a single leaf has none) and coordinates below 2^24
+  if (!s->tree_wide[FK_TREE_SAH] || s->root_is_leaf || !s->filter_ok) return FK_OK;
+  const uint32_t nn = s->node_count, blocks = (nn + 255) / 256;
+  struct {
+    float pad;
+    uint32_t unused;
+    unsigned long long reach;
+  } got = {}, *words = nullptr;
+  const size_t chain_bytes = 2 * sizeof(float4) * (size_t)nn;
+  int rc = fk_dev_alloc(ctx, (void**)&words, sizeof(got));
+  if (rc == FK_OK) rc = fk_dev_alloc(ctx, (void**)&s->chain_box, chain_bytes);
+  cudaError_t e = cudaSuccess;
+  if (rc == FK_OK) e = cudaMemsetAsync(words, 0, sizeof(got), ctx->stream);
+  if (rc == FK_OK && e == cudaSuccess) {
+    map_pad_kernel<<<blocks, 256, 0, ctx->stream>>>(s->node_lo, s->node_hi, s->node_jump, s->pos4, s->tri_rec, nn,
+                                                    (uint32_t*)&words->pad, s->chain_box);
+    rc = fk_after_launch(ctx, "map_pad_kernel");
+  }
+  if (rc == FK_OK && e == cudaSuccess) {
+    map_reach_kernel<<<blocks, 256, 0, ctx->stream>>>(s->node_lo, s->node_hi, nn, &words->pad, &words->reach);
+    rc = fk_after_launch(ctx, "map_reach_kernel");
+  }
+  if (rc == FK_OK && e == cudaSuccess)
+    e = cudaMemcpyAsync(&got, words, sizeof(got), cudaMemcpyDeviceToHost, ctx->stream);
+  if (rc == FK_OK && e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  fk_dev_free(ctx, words);
+  if (rc == FK_OK && e != cudaSuccess) rc = fk_cuda_fail(ctx, e, "mapping bound");
+  if (rc != FK_OK) return rc;  // the scene, and what it holds by now, goes back
+  s->map_pad = got.pad;
+  s->map_reach = (float)got.reach / 16.0f / (float)s->leaf_count;
+  s->map_tree = got.pad <= FLT_MAX && s->map_reach <= kMaxMapReach;
+  if (s->map_tree) {
+    s->bytes += chain_bytes;
+  } else {
+    fk_dev_free(ctx, s->chain_box);
+    s->chain_box = nullptr;
+  }
+  return FK_OK;
 }
 
 // One axis of the padded slab test: value of a face f is fma(f, inv, -ol) for
@@ -2195,11 +2258,11 @@ __device__ bool map_line(const SceneDev& s, f3 o, f3 d, float max_d, float& t, u
                            fmaxf(fabsf(RL.z), fabsf(RH.z)));
   const float far = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fabsf(o.z));
   const float len = fmaxf(fmaxf(fabsf(d.x), fabsf(d.y)), fabsf(d.z));
-  const float M = fmaxf(root, far), bound = __ldg(s.map_pad);
+  const float M = fmaxf(root, far);
   // sums so that a NaN in any component fails (fmaxf drops it)
   const bool finite = fabsf(o.x) + fabsf(o.y) + fabsf(o.z) < 5.0e7f && fabsf(d.x) + fabsf(d.y) + fabsf(d.z) < 4.0f;
-  if (!(finite && M < 16777216.0f && len >= 0.5f && bound <= 0.05f * root)) return false;
-  const float pad = __fadd_rn(bound, __fmul_rn(M, 7.62939453e-06f));  // 128 u
+  if (!(finite && M < 16777216.0f && len >= 0.5f)) return false;
+  const float pad = __fadd_rn(s.map_pad, __fmul_rn(M, 7.62939453e-06f));  // 128 u
   f3 inv, ol, oh;
   line_axis(o.x, d.x, pad, inv.x, ol.x, oh.x);
   line_axis(o.y, d.y, pad, inv.y, ol.y, oh.y);
@@ -2287,11 +2350,12 @@ __device__ bool map_line(const SceneDev& s, f3 o, f3 d, float max_d, float& t, u
 }
 
 // max_d: the walks' initial closest distance (FLT_MAX in the shaders); a
-// miss writes t = FLT_MAX whatever it is.  TREE: map_line first.
-template <int CULL, bool TREE>
+// miss writes t = FLT_MAX whatever it is.  TREE: map_line first; COUNT: adds up
+// the texels it answers.
+template <int CULL, bool TREE, bool COUNT = false>
 __global__ void __launch_bounds__(128) meshmap_kernel(SceneDev s, const float4* __restrict__ pix, float max_d,
                                                       uint32_t offset, uint32_t count, float4* __restrict__ coords,
-                                                      uint32_t* __restrict__ tidx) {
+                                                      uint32_t* __restrict__ tidx, uint32_t* __restrict__ by_tree) {
   uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= count) return;
   uint32_t g = offset + j;
@@ -2310,6 +2374,8 @@ __global__ void __launch_bounds__(128) meshmap_kernel(SceneDev s, const float4* 
       t = fminf(t, walk_twoside(s, p, d, t, id, w));
       t = fminf(t, walk_twoside(s, p, neg(d), t, id, w));
     }
+  } else if (COUNT) {
+    atomicAdd(by_tree, 1u);
   }
   if (id == kMiss) t = FLT_MAX;
   coords[g] = make_float4(t, w.x, w.y, w.z);
@@ -2317,14 +2383,13 @@ __global__ void __launch_bounds__(128) meshmap_kernel(SceneDev s, const float4* 
 }
 
 int launch_meshmap(fk_ctx* ctx, const fk_scene* s, const fk_texel_map* m, int cull, float max_d, uint32_t offset,
-                   uint32_t count, float4* coords, uint32_t* tidx) {
+                   uint32_t count, float4* coords, uint32_t* tidx, uint32_t* by_tree) {
   if (count == 0) return FK_OK;
   uint32_t blocks = (count + 127) / 128;
-  // a rebuilt tree (kept only where it fits the stack; a single leaf has none) and coordinates below 2^24
-  const bool tree = s->tree_wide[FK_TREE_SAH] && !s->root_is_leaf && s->filter_ok;
-  auto kern = cull ? (tree ? meshmap_kernel<1, true> : meshmap_kernel<1, false>)
-                   : (tree ? meshmap_kernel<0, true> : meshmap_kernel<0, false>);
-  kern<<<blocks, 128, 0, ctx->stream>>>(dev_of(s), m->pix, max_d, offset, count, coords, tidx);
+  auto kern = cull ? (s->map_tree ? meshmap_kernel<1, true> : meshmap_kernel<1, false>)
+                   : (s->map_tree ? meshmap_kernel<0, true> : meshmap_kernel<0, false>);
+  if (by_tree && s->map_tree) kern = cull ? meshmap_kernel<1, true, true> : meshmap_kernel<0, true, true>;
+  kern<<<blocks, 128, 0, ctx->stream>>>(dev_of(s), m->pix, max_d, offset, count, coords, tidx, by_tree);
   return fk_after_launch(ctx, "meshmap_kernel");
 }
 

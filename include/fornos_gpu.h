@@ -650,6 +650,15 @@ int fk_diag_traversal_profile(fk_ctx* ctx, const fk_scene* scene, const fk_buf* 
                               const fk_sample_params* params, const fk_buf* samples4, uint32_t offset, uint32_t count,
                               int traverse, uint64_t* counters);
 
+/* No counterpart in the reference.  How fk_meshmap maps this scene: by one
+ * traversal of the surface-area tree where a bound on the hits' rounding allows
+ * it, by the reference's two skip-pointer walks otherwise (same results).
+ * Maps all of `map` and returns the number of texels the tree answered (0: the
+ * scene takes the walks) and, in reach (may be NULL), how many leaves the bound
+ * makes a ray meet on average (infinite without a bound, 0 without a tree). */
+int fk_diag_meshmap_routes(fk_ctx* ctx, const fk_scene* scene, const fk_texel_map* map, int cull_backfaces,
+                           float max_dist, uint32_t* tree_texels, float* reach);
+
 /* No counterpart in the reference.  An inner tree of the scene as resident on
  * the device (FK_TREE_REFERENCE or FK_TREE_SAH): its 2-wide records, 16 words
  * each (floats 0-3 / 4-7: the left / right child's x and y bounds, 8-9 /

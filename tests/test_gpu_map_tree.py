@@ -92,6 +92,35 @@ def test_tree_route_equals_walks(name, cull):
     ctx.check()
 
 
+@pytest.mark.parametrize("angle,tree", [(None, True), (0.3, True), (1e-2, True), (1e-3, True), (2.6e-4, False),
+                                        (2e-4, False)])
+def test_route_follows_the_bound(angle, tree):
+    """One thin triangle widens the bound of the whole scene: the tree route is
+    left where it would meet many more leaves, and where there is no bound."""
+    quads = 200
+    m = W.grid_plane(quads, heights=0.002 * np.random.default_rng(1).uniform(0, 1, (quads + 1) ** 2))
+    if angle is not None:
+        nv, e = len(m.positions), 2.0 ** 0.5
+        pos = np.concatenate([m.positions, [[0, 0, -0.5], [1, 1, -0.5], [1, 1, -0.5 + e * angle]]])
+        m = W.MeshArrays(pos, m.texcoords[:1], [[0, 0, 1]],
+                         np.stack([np.arange(nv + 3), np.zeros(nv + 3), np.zeros(nv + 3)], -1),
+                         np.concatenate([m.triangles, [[nv, nv + 1, nv + 2]]]))
+    ctx = api.Context(0)
+    scene = api.Scene.build(ctx, api.Mesh(m))
+    n = 1000
+    o, d = np.zeros((n, 3)), np.tile([[0.0, 0.0, 1.0]], (n, 1))
+    o[:, :2] = np.random.default_rng(2).uniform(0, 1, (n, 2))
+    pix = np.zeros((n, 8), np.float32)
+    pix[:, 0:3], pix[:, 4:7] = o, d
+    tmap = api.TexelMap.from_host(ctx, n, 1, pix, np.zeros((n, 12), np.float32), np.arange(n))
+    texels, reach = api.meshmap_routes(ctx, scene, tmap, True)
+    assert texels > 0.9 * n if tree else texels == 0
+    assert reach >= 1.0 and np.isinf(reach) == (angle == 2e-4)
+    c1, t1 = mapped(ctx, scene, o, d, True, api.FLT_MAX)
+    c8, t8 = mapped(ctx, scene, o, 8 * d, True, api.FLT_MAX)
+    assert np.array_equal(t1, t8) and np.array_equal(bits(c1[:, 0]), bits(8 * c8[:, 0]))
+
+
 @pytest.mark.parametrize("cull", [True, False])
 @pytest.mark.parametrize("seed", range(4))
 def test_flat_face_outside_its_ancestors_rounded_box(cull, seed):
