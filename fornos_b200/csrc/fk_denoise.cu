@@ -137,9 +137,7 @@ __device__ __forceinline__ float over_spacing(float v, const Centre& c) {
 
 // The 10 features of neighbour j (< 25, row-major over the 5 x 5 window) of
 // the texel at pixel p with centre terms c; zeros outside the texture, without
-// a mapping hit, or for p = kNoTexel.  EXACT: IEEE divisions (the rows that a
-// caller keeps); else over_spacing.
-template <bool EXACT>
+// a mapping hit, or for p = kNoTexel.
 __device__ __forceinline__ void neighbour_features(const float4* __restrict__ f0, const float4* __restrict__ f1,
                                                    const float4* __restrict__ f2, uint32_t w, uint32_t h, uint32_t p,
                                                    const Centre& c, int j, float (&v)[10]) {
@@ -155,9 +153,41 @@ __device__ __forceinline__ void neighbour_features(const float4* __restrict__ f0
   v[1] = a.y;
   v[2] = a.z;
   if (c.spacing > 0.0f) {
-    v[3] = clamp4(EXACT ? (b.x - c.px) / c.spacing : over_spacing(b.x - c.px, c));
-    v[4] = clamp4(EXACT ? (b.y - c.py) / c.spacing : over_spacing(b.y - c.py, c));
-    v[5] = clamp4(EXACT ? (b.z - c.pz) / c.spacing : over_spacing(b.z - c.pz, c));
+    v[3] = clamp4(over_spacing(b.x - c.px, c));
+    v[4] = clamp4(over_spacing(b.y - c.py, c));
+    v[5] = clamp4(over_spacing(b.z - c.pz, c));
+  }
+  v[6] = n.x;
+  v[7] = n.y;
+  v[8] = b.w;
+  v[9] = 1.0f;
+}
+
+// The same with IEEE divisions, a lane per neighbour (the rows that a caller
+// keeps): the centre's terms are loaded behind the coverage test, which saves
+// them for uncovered neighbours (hoisted: 0.349 -> 0.359 ms for the rows of 1024 x
+// 1024 texels).
+__device__ __forceinline__ void neighbour_features_exact(const float4* __restrict__ f0, const float4* __restrict__ f1,
+                                                         const float4* __restrict__ f2, uint32_t w, uint32_t h,
+                                                         uint32_t p, int j, float (&v)[10]) {
+#pragma unroll
+  for (int k = 0; k < 10; ++k) v[k] = 0.0f;
+  if (p == kNoTexel) return;
+  const int cx = (int)(p % w), cy = (int)(p / w);
+  const int x = cx + j % 5 - 2, y = cy + j / 5 - 2;
+  if (x < 0 || y < 0 || x >= (int)w || y >= (int)h) return;
+  const uint32_t q = (uint32_t)y * w + (uint32_t)x;
+  const float4 a = __ldg(f0 + q);
+  if (!(a.w > 0.0f)) return;
+  const float4 c = __ldg(f1 + p), b = __ldg(f1 + q), n = __ldg(f2 + q);
+  const float spacing = __ldg(f2 + p).z;
+  v[0] = a.x;
+  v[1] = a.y;
+  v[2] = a.z;
+  if (spacing > 0.0f) {
+    v[3] = clamp4((b.x - c.x) / spacing);
+    v[4] = clamp4((b.y - c.y) / spacing);
+    v[5] = clamp4((b.z - c.z) / spacing);
   }
   v[6] = n.x;
   v[7] = n.y;
@@ -172,7 +202,7 @@ __device__ __forceinline__ void assemble_row(const float4* __restrict__ f0, cons
                                              int lane, uint32_t* dst) {
   if (lane < 25) {
     float v[10];
-    neighbour_features<true>(f0, f1, f2, w, h, p, centre_of(f1, f2, w, p), lane, v);
+    neighbour_features_exact(f0, f1, f2, w, h, p, lane, v);
 #pragma unroll
     for (int k = 0; k < 5; ++k) dst[5 * lane + k] = pack2(v[2 * k], v[2 * k + 1]);
   } else if (lane == 25) {
@@ -230,6 +260,19 @@ __device__ __forceinline__ void load_forward_weights(const Smem& s, const DnWeig
   copy_words((uint32_t*)s.w3, HS / 2, (const uint32_t*)wt.w3, kHidden / 2, 8, kHidden / 2);
 }
 
+// B fragments of units 8 j .. 8 j + 15 and inputs 16 kk .. 16 kk + 15: both K halves of the first eight units, then
+// of the other eight.  LDM: one ldmatrix, which pays in the training kernel's serial chain; inference, with two CTAs an
+// SM and more instructions to hide them behind, reads word by word (0.380 -> 0.374 ms for 1M rows).
+template <bool LDM>
+__device__ __forceinline__ void weights4(const __nv_bfloat16* w, int stride, int j, int kk, int lane, uint32_t (&b)[4]) {
+  if (LDM) {
+    ldm4(w + (8 * j + (lane & 7) + ((lane & 16) >> 1)) * stride + 16 * kk + (lane & 8), b);
+  } else {
+    const uint32_t* r = (const uint32_t*)(w + (8 * j + (lane >> 2)) * stride) + 8 * kk + (lane & 3);
+    b[0] = r[0], b[1] = r[4], b[2] = r[4 * stride], b[3] = r[4 * stride + 4];
+  }
+}
+
 // Forward pass of one warp's 16 rows (rows r0 .. r0+15 of the tile in s.x).
 // y: network outputs in the C-fragment layout (column 2t + (c & 1), row
 // g + 8 (c >> 1)); only columns 0..3 are meaningful.  TRAIN keeps the GELU
@@ -246,14 +289,13 @@ __device__ __forceinline__ void forward16(const Smem& s, const float* __restrict
     for (int c = 0; c < 4; ++c) acc[j][c] = 0.0f;
   const uint32_t* xr = (const uint32_t*)(s.x + (r0 + g) * XS);
   const uint32_t* xr8 = (const uint32_t*)(s.x + (r0 + g + 8) * XS);
-  const int brow = (lane & 7) + ((lane & 16) >> 1), bcol = lane & 8;  // this lane's row of an ldm4 of weights
 #pragma unroll 4
   for (int kk = 0; kk < kK1 / 16; ++kk) {
     const uint32_t x0 = xr[8 * kk + t], x1 = xr8[8 * kk + t], x2 = xr[8 * kk + 4 + t], x3 = xr8[8 * kk + 4 + t];
 #pragma unroll
     for (int j = 0; j < 8; j += 2) {
       uint32_t b[4];  // units 8 j: both K halves, units 8 j + 8: both K halves
-      ldm4(s.w1 + (8 * j + brow) * XS + 16 * kk + bcol, b);
+      weights4<TRAIN>(s.w1, XS, j, kk, lane, b);
       mma16816(acc[j], x0, x1, x2, x3, b[0], b[1]);
       mma16816(acc[j + 1], x0, x1, x2, x3, b[2], b[3]);
     }
@@ -281,7 +323,7 @@ __device__ __forceinline__ void forward16(const Smem& s, const float* __restrict
 #pragma unroll
     for (int j = 0; j < 8; j += 2) {
       uint32_t b[4];
-      ldm4(s.w2 + (8 * j + brow) * HS + 16 * kk + bcol, b);
+      weights4<TRAIN>(s.w2, HS, j, kk, lane, b);
       mma16816(acc[j], a1[kk][0], a1[kk][1], a1[kk][2], a1[kk][3], b[0], b[1]);
       mma16816(acc[j + 1], a1[kk][0], a1[kk][1], a1[kk][2], a1[kk][3], b[2], b[3]);
     }
@@ -1001,7 +1043,7 @@ __global__ void __launch_bounds__(tc::kThreads, tc::kCtasPerSm) dn_apply_tc_kern
 #pragma unroll 2
       for (uint32_t j = part; j < 25; j += 4) {
         float v[10];
-        neighbour_features<false>(a.f0, a.f1, a.f2, a.w, a.h, px, c, (int)j, v);
+        neighbour_features(a.f0, a.f1, a.f2, a.w, a.h, px, c, (int)j, v);
         *(uint4*)(sm + tc::kA1 + tc::core_off(r, 8 * j, 256)) =
             make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
         *(uint32_t*)(sm + tc::kA1 + tc::core_off(r, 200 + 2 * j, 256)) = pack2(v[8], v[9]);
