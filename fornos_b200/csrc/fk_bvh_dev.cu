@@ -14,9 +14,10 @@
 // node's bins), one thread per node runs the host's split sweep, blocks reduce
 // the two sides' boxes and count the left side, and the host turns the counts
 // into offsets for a stable partition.  Nodes of at most kSmall triangles are
-// built by one warp each, in the host recursion's order, in shared memory.  The top of the tree stays on the host, which recomputes its boxes
-// from the children after the subtrees are done and assigns the preorder
-// indices; kernels then write the flattened records and the corners.
+// built by one warp each, in the host recursion's order, in shared memory.  The
+// top of the tree stays on the host, which recomputes its boxes from the
+// children after the subtrees are done and assigns the preorder indices;
+// kernels then write the flattened records and the corners.
 #include <algorithm>
 #include <vector>
 
@@ -1100,11 +1101,8 @@ int build_bvh_device(fk_ctx* ctx, const fk_mesh* mesh, uint32_t max_tris, uint32
     bvh_small_roots_kernel<<<(nsm + 127) / 128, 128, 0, st>>>(d_small, nsm, dnodes, d_roots);
     if ((rc = fk_after_launch(ctx, "bvh subtree roots")) != FK_OK) return done2(rc);
     e = cudaMemcpyAsync(roots.data(), d_roots, sizeof(DNode) * nsm, cudaMemcpyDeviceToHost, st);
-    uint32_t status = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&status, d_status, 4, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return done2(fk_cuda_fail(ctx, e, "device BVH build: subtrees"));
-    if (status) return done2(fk_fail(ctx, FK_ERR_DEVICE, "device BVH build: subtree check failed"));
   }
   // top of the tree: boxes from the children (Src/bvh.cpp:266-276), sizes, preorder
   auto kid_box = [&](int32_t r, float c[3], float s[3], uint32_t& size) {
