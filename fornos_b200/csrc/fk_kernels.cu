@@ -2103,8 +2103,9 @@ __device__ float walk_twoside(const SceneDev& s, f3 o, f3 d, float mint, uint32_
 // |d| < 2^-100 has 1 / d replaced by 2^100 (t < 2^27, so the ray moves less than
 // 2^-73 along it, and the padded faces are as good as infinitely far or behind).
 // map_pad_kernel gives an infinite bound where this does not hold: s below
-// 2^-24, edges outside [2^-25, 2^25], a triangle outside its leaf's box or the
-// root's coordinates (an uploaded scene); a triangle whose normal is NaN is
+// 2^-24, edges outside [2^-25, 2^25], a triangle further than that 8 u M' outside
+// its leaf's box or the root's coordinates (an uploaded scene: a build's own
+// boxes, rounded from centre and half size, end an ulp short of a corner at most); a triangle whose normal is NaN is
 // never hit.  Scenes without a bound, or with one that makes the traversal meet
 // too many leaves (kMaxMapReach), take the walks altogether; directions far from
 // unit length and origins from 2^24 up take them too.
@@ -2160,7 +2161,7 @@ __global__ void map_pad_kernel(const float4* __restrict__ lo, const float4* __re
       const double s = (x * x + y * y + z * z) / (d00 * d11);
       const double edge2 = 8.8817841970012523e-16;  // 2^-50
       const bool ok = s >= 5.9604644775390625e-08 && d00 >= edge2 && d11 >= edge2 && d00 <= 1.0 / edge2 &&
-                      d11 <= 1.0 / edge2 && fabsf(a.x) <= M && fabsf(a.y) <= M && fabsf(a.z) <= M;
+                      d11 <= 1.0 / edge2 && fabsf(a.x) <= M + tol && fabsf(a.y) <= M + tol && fabsf(a.z) <= M + tol;
       const double q = (sqrt(d00) + sqrt(d11)) * (2.1e-5 + 17.0 * 5.9604644775390625e-08 / sqrt(s));
       p = fmaxf(p, ok && q <= 0.05 * M ? __double2float_ru(q) : inf);
     }

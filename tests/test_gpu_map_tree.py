@@ -2,7 +2,7 @@
 bit.  A direction eight times as long takes the walks (the tree route asks for
 about unit length) and every operation on it is the same but for an exact power
 of two, so both routes run on the same rays and distances differ by that
-factor alone."""
+factor alone.  That the tree answered the unit directions is counted."""
 import numpy as np
 import pytest
 
@@ -13,17 +13,33 @@ from tests.cases import bits
 pytestmark = pytest.mark.gpu
 
 
-def soup(n, seed, size):
-    """Triangles of all shapes: ordinary ones, slivers, repeated corners,
-    collinear corners, identical triangles, one as large as the scene."""
+def soup(n, seed, size, thin=None, scale=1.0, shift=(0.0, 0.0, 0.0), slivers=False):
+    """Triangles of all shapes: ordinary ones, thin ones (down to the angle
+    `thin`), repeated corners, collinear corners, identical triangles, one as
+    large as the scene; with `slivers` thinner than any bound allows."""
     rng = np.random.default_rng(seed)
     c = rng.uniform(-1, 1, (n, 1, 3))
     p = (c + size * rng.normal(size=(n, 3, 3))).astype(np.float32)
-    p[1::7, 2] = p[1::7, 1] + (p[1::7, 0] - p[1::7, 1]) * np.float32(1e-3) + np.float32(1e-6)
+    if slivers:
+        p[1::7, 2] = p[1::7, 1] + (p[1::7, 0] - p[1::7, 1]) * np.float32(1e-3) + np.float32(1e-6)
+        p[3::7, 2] = 0.5 * (p[3::7, 0] + p[3::7, 1])
+    else:
+        v0, v1 = p[:, 1] - p[:, 0], p[:, 2] - p[:, 0]
+        up = np.cross(v0, v1)
+        up /= np.linalg.norm(up, axis=1, keepdims=True)
+        across = np.cross(up, v0)  # of v0's length, at a right angle to it in the triangle's plane
+        sin = np.linalg.norm(np.cross(v0, v1), axis=1) / (np.linalg.norm(v0, axis=1) * np.linalg.norm(v1, axis=1))
+        p[:, 2] = np.where((sin < 0.1)[:, None], p[:, 0] + across, p[:, 2])
+        if thin:
+            a = np.exp(rng.uniform(np.log(thin), 0, n))[:, None]
+            p[1::7, 2] = (p[:, 0] + v0 * np.cos(a) + across * np.sin(a))[1::7]
+        # collinear to the last bit: grid points with the third corner twice as far as the second
+        q, g = (p[3::7, 0] * 64).round() / 64, (v0[3::7] * 256).round() / 256
+        p[3::7] = np.stack([q, q + g, q + 2 * g], 1)
     p[2::7, 2] = p[2::7, 1]
-    p[3::7, 2] = 0.5 * (p[3::7, 0] + p[3::7, 1])
     p[4::14] = p[4]
     p[-1] = [[-1, -1, 0], [1, -1, 0], [0, 1, 0]]
+    p = p * np.float32(scale) + np.asarray(shift, np.float32)
     tri = np.arange(3 * n).reshape(-1, 3)
     return W.MeshArrays(p.reshape(-1, 3), np.zeros((1, 2)), np.tile([[0, 0, 1]], (3 * n, 1)),
                         np.stack([np.arange(3 * n), np.zeros(3 * n), np.arange(3 * n)], -1), tri)
@@ -34,9 +50,14 @@ MESHES = {
     "heights": lambda: W.plane_pair(seed=4, hi_quads=64, bumps=20)[1],
     "flat": lambda: W.grid_plane(32),                                 # every hit lies in its leaf's box face
     "soup": lambda: soup(4000, 5, 0.02),
+    "thin_soup": lambda: soup(4000, 9, 0.02, thin=4e-4),
     "coarse_soup": lambda: soup(300, 6, 0.4),
-    "two": lambda: W.grid_plane(1),
+    "small_soup": lambda: soup(1000, 10, 0.05, scale=2.0 ** -9, shift=(0.5, -0.25, 0.125)),
+    "large_soup": lambda: soup(1000, 11, 0.05, scale=64.0, shift=(100.0, -300.0, 50.0)),
+    "two": lambda: W.grid_plane(1),                             # a single leaf has no tree
     "nine": lambda: soup(9, 7, 0.3),
+    "slivers": lambda: soup(4000, 5, 0.02, slivers=True),       # no bound: the walks throughout
+    "nine_slivers": lambda: soup(9, 7, 0.3, slivers=True),
 }
 
 
@@ -60,11 +81,16 @@ def rays(mesh, n, seed):
     return o.astype(np.float32), d.astype(np.float32)
 
 
-def mapped(ctx, scene, o, d, cull, max_d):
+def texel_map(ctx, o, d):
     n = len(o)
     pix = np.zeros((n, 8), np.float32)
     pix[:, 0:3], pix[:, 4:7] = o, d
-    tmap = api.TexelMap.from_host(ctx, n, 1, pix, np.zeros((n, 12), np.float32), np.arange(n))
+    return api.TexelMap.from_host(ctx, n, 1, pix, np.zeros((n, 12), np.float32), np.arange(n))
+
+
+def mapped(ctx, scene, o, d, cull, max_d):
+    n = len(o)
+    tmap = texel_map(ctx, o, d)
     coords, tidx = ctx.buffer(16 * n), ctx.buffer(4 * n)
     api.meshmap(ctx, scene, tmap, cull, coords, tidx, max_dist=max_d)
     return coords.download(np.float32, (n, 4)), tidx.download(np.uint32, n)
@@ -84,11 +110,15 @@ def test_tree_route_equals_walks(name, cull):
         c1, t1 = mapped(ctx, scene, o, d, cull, max_d)
         c8, t8 = mapped(ctx, scene, o, 8 * d, cull, max_d if max_d == api.FLT_MAX else max_d / 8)
         hit = t1 != api.MISS
+        by_tree, _ = api.meshmap_routes(ctx, scene, texel_map(ctx, o, d), cull, max_d)
+        walked, _ = api.meshmap_routes(ctx, scene, texel_map(ctx, o, 8 * d), cull, max_d)
+        assert walked == 0
+        assert by_tree == 0 if "slivers" in name or name == "two" else by_tree > 0.8 * len(o)
         assert np.array_equal(t1, t8)
         # as bits: a texel on a triangle seen from behind maps to -0
         assert np.array_equal(bits(c1[hit, 0]), bits(8 * c8[hit, 0]))
         assert np.array_equal(bits(c1[:, 1:]), bits(c8[:, 1:]))
-        assert hit.sum() > 100 or name in ("two", "nine", "flat")
+        assert hit.sum() > 100 or name in ("two", "nine", "nine_slivers", "flat")
     ctx.check()
 
 
@@ -110,10 +140,7 @@ def test_route_follows_the_bound(angle, tree):
     n = 1000
     o, d = np.zeros((n, 3)), np.tile([[0.0, 0.0, 1.0]], (n, 1))
     o[:, :2] = np.random.default_rng(2).uniform(0, 1, (n, 2))
-    pix = np.zeros((n, 8), np.float32)
-    pix[:, 0:3], pix[:, 4:7] = o, d
-    tmap = api.TexelMap.from_host(ctx, n, 1, pix, np.zeros((n, 12), np.float32), np.arange(n))
-    texels, reach = api.meshmap_routes(ctx, scene, tmap, True)
+    texels, reach = api.meshmap_routes(ctx, scene, texel_map(ctx, o, d), True)
     assert texels > 0.9 * n if tree else texels == 0
     assert reach >= 1.0 and np.isinf(reach) == (angle == 2e-4)
     c1, t1 = mapped(ctx, scene, o, d, True, api.FLT_MAX)
