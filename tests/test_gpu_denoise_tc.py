@@ -89,3 +89,28 @@ def test_engine_choice_is_validated(ctx):
     dn = api.Denoiser(ctx)
     with pytest.raises(api.FornosError):
         dn.set_engine(7)
+
+
+def test_apply_against_forward_on_the_same_rows(ctx):
+    """An image's input rows are summed in another order than rows that a caller
+    keeps, and their quotients come from a reciprocal: the two may differ as the
+    engines do, by accumulation order and the flips of a bf16 rounding."""
+    rng = np.random.default_rng(3)
+    w, h = 61, 40
+    n = w * h
+    image = rng.uniform(-1, 1, (3, n, 4)).astype(np.float32)
+    image[0, :, 3] = rng.uniform(0, 1, n) > 0.1
+    image[2, :, 2] = rng.uniform(0.2, 1.0, n)
+    tm = api.TexelMap.from_host(ctx, w, h, np.zeros((n, 8)), np.zeros((n, 12)), np.arange(n))
+    img, tidx = ctx.upload(image), ctx.upload(np.zeros(n, np.uint32))
+    ao = rng.uniform(0.3, 0.7, n).astype(np.float32)
+    bn = rng.normal(size=(n, 3)).astype(np.float32)
+    dn = api.Denoiser(ctx, params(4))
+    out_ao, out_bn = ctx.buffer(4 * n), ctx.buffer(12 * n)
+    dn.apply(tm, img, tidx, ctx.upload(ao), ctx.upload(bn), out_ao, out_bn)
+    rows = api.denoise_rows(ctx, img, w, h, ctx.upload(np.arange(n, dtype=np.uint32)), n)
+    y = dn.forward(rows, n).download(np.float32, (n, 4)).astype(np.float64)
+    ctx.check()
+    close(out_ao.download(np.float32, n), np.clip(ao + y[:, 0], 0, 1))
+    v = bn + y[:, 1:]
+    close(out_bn.download(np.float32, (n, 3)), v / np.linalg.norm(v, axis=1, keepdims=True))

@@ -1,7 +1,9 @@
 """Rays started at their own triangle's leaf (the 2-wide ordered traversal)
 against the skip-pointer walk: the occluder counts of AO do not depend on the
 order in which leaves are visited, so both are equal exactly, for any triangle
-a texel names, in either inner tree, alone and in a batch."""
+a texel names, in either inner tree, alone and in a batch.  Thickness takes the
+closest hit, where a hit in the face of its leaf's box may be met or not by that
+order: equal but for single texels."""
 import numpy as np
 import pytest
 
@@ -77,3 +79,30 @@ def test_staged_records_of_every_size(top):
         got.append(hits.download(np.uint32, n))
     ctx.check()
     assert got[0].max() > 0 and np.array_equal(*got)
+
+
+@pytest.mark.parametrize("shape", ["heights", "sphere"])
+@pytest.mark.parametrize("tree", [api.TREE_SAH, api.TREE_REFERENCE])
+def test_closest_hits_from_the_own_leaf(shape, tree):
+    ctx = api.Context(0)
+    mesh = api.Mesh(flat(64, 2) if shape == "heights" else W.sphere_pair(seed=2, hi_seg=(96, 48))[1])
+    mesh.compute_vertex_normals()
+    scene = api.Scene.build(ctx, mesh)
+    scene.set_tree(tree)
+    nt, n, hi = scene.info()["corner_count"] // 3, 3000, 3.0
+    rng = np.random.default_rng(7)
+    coords = np.zeros((n, 4), np.float32)
+    coords[:, 1:] = rng.dirichlet((1, 1, 1), n)
+    cb, tb = ctx.upload(coords), ctx.upload((3 * rng.integers(0, nt, n)).astype(np.uint32))
+    table = ctx.upload(api.samples_cosine(SPP, 16, 3))
+    got = []
+    for traverse in (api.TRAVERSE_ORDERED, api.TRAVERSE_SKIP):
+        out, hits = ctx.buffer(4 * n), ctx.buffer(4 * n)
+        api.hemisphere(ctx, scene, cb, tb, api.THICK, SPP, LO, hi, table, out, None, hits, None, 0, n, 16, traverse)
+        got.append((out.download(np.float32, n), hits.download(np.uint32, n)))
+    ctx.check()
+    assert 0.2 < (got[1][1] > 0).mean()
+    # a hit met by one order alone changes its texel's mean of SPP distances by at most hi / SPP
+    differ = got[0][0] != got[1][0]
+    assert differ.mean() <= 1e-3 and np.all(np.abs(got[0][0] - got[1][0]) <= 2 * hi / SPP)
+    assert np.array_equal(got[0][1][~differ], got[1][1][~differ])
