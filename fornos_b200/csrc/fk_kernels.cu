@@ -2105,7 +2105,9 @@ __device__ float walk_twoside(const SceneDev& s, f3 o, f3 d, float mint, uint32_
 // map_pad_kernel gives an infinite bound where this does not hold: s below
 // 2^-24, edges outside [2^-25, 2^25], a triangle further than that 8 u M' outside
 // its leaf's box or the root's coordinates (an uploaded scene: a build's own
-// boxes, rounded from centre and half size, end an ulp short of a corner at most); a triangle whose normal is NaN is
+// boxes, rounded from centre and half size, end an ulp short of a corner at most),
+// leaves whose corners do not ascend (an uploaded scene: among hits at one
+// distance the walks keep the first they meet); a triangle whose normal is NaN is
 // never hit.  Scenes without a bound, or with one that makes the traversal meet
 // too many leaves (kMaxMapReach), take the walks altogether; directions far from
 // unit length and origins from 2^24 up take them too.
@@ -2143,6 +2145,10 @@ __global__ void map_pad_kernel(const float4* __restrict__ lo, const float4* __re
         }
       }
       if (steps > kMaxChain) p = inf;  // an uploaded tree of extreme depth: the walks
+      // the smallest corner is the one met first only where the leaves' corners ascend (an uploaded tree may differ)
+      uint32_t before = i;
+      while (before > 0 && as_u32(lo[before - 1].w) == as_u32(hi[before - 1].w)) --before;
+      if (before > 0 && as_u32(hi[before - 1].w) > as_u32(L.w)) p = inf;
       // A flat leaf at an ancestor's rounded face can lie an ulp outside it.  Nothing is then in both boxes, and the
       // box test would swap the faces and report an entry before the ancestor's: a box that no ray enters instead.
       if (cl.x > ch.x || cl.y > ch.y || cl.z > ch.z) cl.x = ch.x = cl.y = ch.y = cl.z = ch.z = __int_as_float(0x7fffffff);

@@ -122,6 +122,41 @@ def test_tree_route_equals_walks(name, cull):
     ctx.check()
 
 
+@pytest.mark.parametrize("cull", [True, False])
+def test_leaves_in_another_order_than_their_corners(cull):
+    """Among hits at one distance the walks keep the first they meet, which is
+    the smallest corner only where the leaves' corners ascend: an uploaded tree
+    whose leaves name them in descending order, on the edges between leaves."""
+    quads, n = 16, 4000
+    mesh = api.Mesh(W.grid_plane(quads))
+    built = api.BVH.create_binary(mesh).flatten(mesh)
+    nodes, pos4, nrm4 = (a.copy() for a in built)
+    order, at = [], 0
+    for i in np.flatnonzero(nodes["end"] > nodes["start"])[::-1]:
+        corners = np.arange(nodes["start"][i], nodes["end"][i])
+        nodes["start"][i], nodes["end"][i] = at, at + len(corners)
+        at += len(corners)
+        order.append(corners)
+    order = np.concatenate(order)
+    turned = (nodes, pos4[order], nrm4[order])
+    ctx = api.Context(0)
+    rng = np.random.default_rng(5)
+    d = np.tile([[0.6, 0.0, 0.8]], (n, 1))
+    # into the plane a little behind a grid line, inside the barycentric slack of the triangles before it
+    at = np.stack([rng.integers(1, quads, n) / quads + rng.uniform(0, 6e-7, n), rng.uniform(0, 1, n), np.zeros(n)], -1)
+    at[::2, 0] = rng.uniform(0, 1, n // 2)  # and anywhere
+    o = (at - 0.25 * d).astype(np.float32)
+    d = d.astype(np.float32)
+    for ascending, arrays in ((True, built), (False, turned)):
+        scene = api.Scene(ctx, *arrays)
+        by_tree, _ = api.meshmap_routes(ctx, scene, texel_map(ctx, o, d), cull)
+        assert by_tree > 0.3 * n if ascending else by_tree == 0
+        c1, t1 = mapped(ctx, scene, o, d, cull, api.FLT_MAX)
+        c8, t8 = mapped(ctx, scene, o, 8 * d, cull, api.FLT_MAX)
+        assert (t1 != api.MISS).mean() > 0.9
+        assert np.array_equal(t1, t8) and np.array_equal(bits(c1[:, 1:]), bits(c8[:, 1:]))
+
+
 @pytest.mark.parametrize("angle,tree", [(None, True), (0.3, True), (1e-2, True), (1e-3, True), (2.6e-4, False),
                                         (2e-4, False)])
 def test_route_follows_the_bound(angle, tree):
