@@ -74,8 +74,8 @@ WORKLOADS = {
 TRAVERSE = {"auto": 0, "ordered": 1, "skip": 2, "ordered4": 3}
 SCHEDULE = {"auto": 0, "static": 0x10, "dynamic": 0x20}
 # DRAM bytes (read + write) per hemisphere-kernel launch from ncu captures, by workload: plane250, one AO+BN
-# trace launch of 968,256 rays (profiles/hemi_trace_kernel_plane250.md); plane2048, the mean of two AO+BN
-# chunk launches of 134,217,728 rays each, 4.42 and 2.91 GB (profiles/hemi_trace_traffic_plane2048.md).
+# trace launch of 968,256 rays; plane2048, the mean of two AO+BN chunk launches of 134,217,728 rays each, 4.42 and
+# 2.91 GB.
 NCU_TRAFFIC = {"plane250": 254.3e6, "plane2048": 3.663e9}
 
 

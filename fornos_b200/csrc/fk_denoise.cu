@@ -425,9 +425,11 @@ struct TrainArgs {
 // One CTA per tile of 128 rows and one tile per SM at the usual batch, so the
 // time is that of one tile's chain: fetch, four dependent layers, gradients.
 // The fetch puts the tile's 128 rows and all weights in flight at once (cp.async;
-// a row id, then its row, sixteen times in a row before), and the operands of
-// the matrix products come from ldmatrix, transposed where the product needs it
-// (2-byte loads before): 23.7 -> 18.8 us at a batch of 16,384.
+// a row id, then its row, sixteen times in a row before).  The weights of the
+// forward pass and dZ1, and both operands of dW1, come from ldmatrix, transposed
+// where the product needs it (dW1's inputs by 2-byte loads before); the forward
+// pass reads its input rows word by word, dW2 and dW3 one operand by 2-byte loads.
+// 23.7 -> 18.8 us at a batch of 16,384.
 __global__ void __launch_bounds__(256, 1) dn_train_kernel(TrainArgs p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __nv_bfloat16* base = (__nv_bfloat16*)smem_raw;

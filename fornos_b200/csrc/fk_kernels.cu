@@ -2097,8 +2097,9 @@ __device__ float walk_twoside(const SceneDev& s, f3 o, f3 d, float mint, uint32_
 // by at most 39 u M' + 7.1 u |p - a| (rounding of t and p, see below) plus
 // |p - a| 16 u / sqrt(s) for the rounded normal, 10.4 u M' more to the ray
 // itself: map_pad = max L (2.1e-5 + 17 u / sqrt(s)); a triangle may stick out of
-// its rounded leaf box by 8 u M', and 128 u leaves 67 u M' for the slab values.  (an and pn: 3.1 u each of a Euclidean norm of at most
-// sqrt(3) M', their difference u, nd 3.1 u of t, p 2 u (t + |p|).)  A slab value is one fused
+// its rounded leaf box by 8 u M', and 128 u leaves 67 u M' for the slab values.
+// (an and pn: 3.1 u each of a Euclidean norm of at most sqrt(3) M', their
+// difference u, nd 3.1 u of t, p 2 u (t + |p|).)  A slab value is one fused
 // multiply-add on face and offset, off by at most 5.1 u M' |1 / d|; an axis with
 // |d| < 2^-100 has 1 / d replaced by 2^100 (t < 2^27, so the ray moves less than
 // 2^-73 along it, and the padded faces are as good as infinitely far or behind).
@@ -2151,7 +2152,10 @@ __global__ void map_pad_kernel(const float4* __restrict__ lo, const float4* __re
       if (before > 0 && as_u32(hi[before - 1].w) > as_u32(L.w)) p = inf;
       // A flat leaf at an ancestor's rounded face can lie an ulp outside it.  Nothing is then in both boxes, and the
       // box test would swap the faces and report an entry before the ancestor's: a box that no ray enters instead.
-      if (cl.x > ch.x || cl.y > ch.y || cl.z > ch.z) cl.x = ch.x = cl.y = ch.y = cl.z = ch.z = __int_as_float(0x7fffffff);
+      if (cl.x > ch.x || cl.y > ch.y || cl.z > ch.z) {
+        const float nan = __int_as_float(0x7fffffff);
+        cl = ch = mk3(nan, nan, nan);
+      }
       chain[2 * (size_t)i] = make_float4(cl.x, cl.y, cl.z, 0.0f);
       chain[2 * (size_t)i + 1] = make_float4(ch.x, ch.y, ch.z, 0.0f);
     }
@@ -2333,7 +2337,8 @@ __device__ bool map_line(const SceneDev& s, f3 o, f3 d, float max_d, float& t, u
         const f3 q = bary_f64(add(o, scale(d, th)), xyz(__ldg(s.pos4 + k)), xyz(__ldg(s.pos4 + k + 1)),
                               xyz(__ldg(s.pos4 + k + 2)));
         if (!bary_ok_map(q)) continue;
-        const float4 cl = __ldg(s.chain_box + 2 * (size_t)(-(cur + 1))), ch = __ldg(s.chain_box + 2 * (size_t)(-(cur + 1)) + 1);
+        const float4* chain = s.chain_box + 2 * (size_t)(-(cur + 1));
+        const float4 cl = __ldg(chain), ch = __ldg(chain + 1);
         const bool visited = ray_box(o, wk ? neg(d) : d, xyz(cl), xyz(ch)) <= at;
         sure = at < best ? visited : sure && visited;
         best = wk ? -th : th;  // the walk's own distance: -0 stays -0

@@ -23,7 +23,10 @@
  * Conventions.  Every function returns FK_OK (0) or a negative FK_ERR_* code;
  * nothing aborts or throws across the ABI.  fk_last_error(ctx) describes the
  * last failure of that context.  Device work is ordered on the context's
- * stream (fk_ctx_set_stream); functions that return host data synchronise it.
+ * stream (fk_ctx_set_stream); functions that return host data synchronise it,
+ * the others may return with work in flight (fk_raster_uv, which waits for its
+ * texel count only, and fk_texel_map_free, whose memory goes back in stream
+ * order, among them), whose errors a later call reports.
  * Handles belong to the context that made them and are freed by their *_free
  * call or by fk_ctx_destroy.  One context per host thread.
  */
@@ -229,7 +232,8 @@ int fk_scene_get_info(const fk_scene* scene, fk_scene_info* out);
  * its leaves' own tests reject), so results stay within the ordered
  * traversal's bar.  Both trees stay resident; choosing the reference's for the
  * first time allocates 8 bytes per triangle (where a ray starts in it).  Mesh
- * mapping does not depend on the choice.  The rebuilt tree is not built when a
+ * mapping does not depend on the choice; where it walks the rebuilt tree the
+ * scene holds 32 bytes per node for it.  The rebuilt tree is not built when a
  * leaf box coordinate is not finite or not below 1e30 in magnitude, nor kept
  * when it is deeper than 48 levels. */
 #define FK_TREE_REFERENCE 0
