@@ -960,6 +960,9 @@ __device__ __forceinline__ bool leaf_phase_warp(const SceneDev& s, const RayPre&
 // down to it, so the siblings the ray may hit are deferred, the root's first (it
 // is popped last), and the leaf is postponed.  Exact for any triangle and any
 // origin: nothing is skipped, the boxes along the way are only taken as hit.
+// With divided box tests rays start at the root: over the reference's tree they
+// reject what the reference's walk rejects, boxes on the way that the ray misses
+// by the rounding of a flat leaf's ancestors included.
 // What it saves: a ray visits 34 inner records from the root on the
 // 2.1M-triangle heightfield, of which 18.5 hold its own origin, at 10 to 11 of
 // a warp's 32 lanes a visit; here the freshly filled lanes test one sibling a
@@ -970,7 +973,7 @@ __device__ __forceinline__ bool leaf_phase_warp(const SceneDev& s, const RayPre&
 // 261k-triangle sphere from 5.59 to 4.74 ms (3.94).
 // TOP: the way down starts in the staged records, whose child refs name staged
 // records, so the siblings deferred there are read from shared memory as well.
-template <bool COUNT, bool FILTER, int S, bool TOP = false>
+template <bool COUNT, int S, bool TOP = false>
 __device__ __forceinline__ void path_start(const float4* __restrict__ wide, const RayPre& rp, const float* ray,
                                            int32_t root, uint64_t path, float hi, OState& st, int32_t* stk,
                                            Tally& tally, const float4* top = nullptr, uint32_t top_base = 0) {
@@ -988,8 +991,8 @@ __device__ __forceinline__ void path_start(const float4* __restrict__ wide, cons
     }
     float entry;
     if (COUNT) tally.box++;
-    const bool h = child_maybe<FILTER, S>(rp, ray, mk3(xy.x, xy.z, second ? z.x : z.z),
-                                          mk3(xy.y, xy.w, second ? z.y : z.w), hi, entry);
+    const bool h = child_maybe<true, S>(rp, ray, mk3(xy.x, xy.z, second ? z.x : z.z),
+                                        mk3(xy.y, xy.w, second ? z.y : z.w), hi, entry);
     if (h) stk[sp] = __float_as_int(second ? w3.x : w3.y);
     sp += h;
     ref = __float_as_int(second ? w3.y : w3.x);
@@ -1031,8 +1034,9 @@ __device__ __forceinline__ bool skip_step(const SceneDev& s, const RayPre& rp, c
 // three times as long: 4 of them, and its loop is not unrolled, which spilled
 // (AO of 200 x 200 texels at 64 spp on 500k triangles: 8 visits unrolled 1.57 ms,
 // with divided box tests 4.66; 4 not unrolled 1.25 and 1.72).  Divided box tests
-// keep their loop rolled for the same reason (2-wide 1.88 against 1.39 ms), the
-// filtered 2-wide visit gains 2 % from the unrolling.
+// keep their loop rolled for the same reason (2-wide, rays from their own leaf,
+// 1.88 against 1.39 ms; from the root 1.56), the filtered 2-wide visit gains 2 %
+// from the unrolling.
 template <int TRAV>
 __host__ __device__ constexpr int inner_visits() {
   return TRAV == FK_TRAVERSE_ORDERED4 ? 4 : 8;
@@ -1112,9 +1116,9 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 512 ? 2 : 1280 / BLOCK) hemi_t
               if (COUNT) tally.box++;
               if (child_hit<FILTER>(rp, o, dir, xyz(L), xyz(H), p.hi, a)) {  // ray_box(o, dir, root) < hi, exactly
                 uint64_t path = 0;
-                if (TRAV == FK_TRAVERSE_ORDERED && p.s.tri_path) path = __ldg(p.s.tri_path + id / 3);
-                if (TRAV == FK_TRAVERSE_ORDERED && path) {
-                  path_start<COUNT, FILTER, BLOCK, TOP>(p.s.wide, rp, myray, TOP ? (int32_t)top_base : 0, path, p.hi,
+                if (TRAV == FK_TRAVERSE_ORDERED && FILTER && p.s.tri_path) path = __ldg(p.s.tri_path + id / 3);
+                if (TRAV == FK_TRAVERSE_ORDERED && FILTER && path) {
+                  path_start<COUNT, BLOCK, TOP>(p.s.wide, rp, myray, TOP ? (int32_t)top_base : 0, path, p.hi,
                                                         st, stk, tally, top_smem, top_base);
                 } else {
                   st.sp = 0;
@@ -1627,9 +1631,9 @@ __global__ void __launch_bounds__(256, FK_BATCH_MIN_BLOCKS) batch_trace_kernel(B
               float aa;
               if (child_hit<FILTER>(rp, o, dir, xyz(L), xyz(H), hi, aa)) {  // ray_box(o, dir, root) < hi, exactly
                 uint64_t path = 0;
-                if (TRAV == FK_TRAVERSE_ORDERED) path = __ldg(s.tri_path + (id + J.corner_base) / 3);
-                if (TRAV == FK_TRAVERSE_ORDERED && path) {
-                  path_start<false, FILTER, 256>(s.wide, rp, myray, J.root2, path, hi, st, stk, tally);
+                if (TRAV == FK_TRAVERSE_ORDERED && FILTER) path = __ldg(s.tri_path + (id + J.corner_base) / 3);
+                if (TRAV == FK_TRAVERSE_ORDERED && FILTER && path) {
+                  path_start<false, 256>(s.wide, rp, myray, J.root2, path, hi, st, stk, tally);
                 } else {
                   st.sp = 0;
                   st.cur = J.root_is_leaf ? kNoRef : (TRAV == FK_TRAVERSE_ORDERED4 ? J.root4 : J.root2);

@@ -299,7 +299,9 @@ typedef struct fk_sample_params {
 #define FK_SCHEDULE_DYNAMIC 0x20 /* lanes refilled with rays from a queue */
 #define FK_SCHEDULE_MASK 0xF0
 /* Divide for every ray-box slab instead of the filtered reciprocal form (the
- * dynamic schedule's default), which takes the same decisions. */
+ * dynamic schedule's default), which takes the same decisions at leaf boxes and
+ * may prune less at inner ones.  Over FK_TREE_REFERENCE the divided 2-wide
+ * traversal finds the hits that the skip walk finds. */
 #define FK_EXACT_BOX_TESTS 0x100
 
 /* Hemisphere sampling for texels [offset, offset + count) (global indices

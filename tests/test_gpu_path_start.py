@@ -106,3 +106,53 @@ def test_closest_hits_from_the_own_leaf(shape, tree):
     differ = got[0][0] != got[1][0]
     assert differ.mean() <= 1e-3 and np.all(np.abs(got[0][0] - got[1][0]) <= 2 * hi / SPP)
     assert np.array_equal(got[0][1][~differ], got[1][1][~differ])
+
+
+def boxes(seed):
+    """Closed boxes of flat, axis-aligned faces: leaves at faces of ancestors whose boxes round inward."""
+    rng = np.random.default_rng(seed)
+    g = W.grid_plane(6)
+    parts = []
+    for lo in rng.uniform(-1, 1, (8, 3)):
+        size = rng.uniform(0.1, 0.8, 3)
+        for axis in range(3):
+            for side in (0, 1):
+                p = np.zeros((len(g.positions), 3))
+                p[:, (axis + 1) % 3], p[:, (axis + 2) % 3], p[:, axis] = g.positions[:, 0], g.positions[:, 1], side
+                parts.append((lo + p * size)[g.triangles])
+    n = 3 * sum(map(len, parts))
+    return W.MeshArrays(np.concatenate(parts).reshape(-1, 3), np.zeros((1, 2)), [[0, 0, 1]],
+                        np.stack([np.arange(n), np.zeros(n), np.zeros(n)], -1), np.arange(n).reshape(-1, 3))
+
+
+@pytest.mark.parametrize("seed", range(3))
+@pytest.mark.parametrize("kind", [api.AO, api.THICK])
+def test_divided_box_tests_over_the_references_tree_equal_the_walk(seed, kind):
+    """They reject exactly what the skip walk rejects, on meshes whose filtered
+    traversal finds hits that the walk does not reach: hit counts are equal."""
+    ctx = api.Context(0)
+    mesh = api.Mesh(boxes(seed))
+    mesh.compute_vertex_normals()
+    scene = api.Scene.build(ctx, mesh)
+    scene.set_tree(api.TREE_REFERENCE)
+    nt, n = scene.info()["corner_count"] // 3, 3000
+    rng = np.random.default_rng(seed)
+    coords = np.zeros((n, 4), np.float32)
+    coords[:, 1:] = rng.dirichlet((1, 1, 1), n)
+    coords[1::3, 1:] = (0.5, 0.5, 0.0)
+    cb, tb = ctx.upload(coords), ctx.upload((3 * rng.integers(0, nt, n)).astype(np.uint32))
+    table = ctx.upload(api.samples_cosine(SPP, 16, 3))
+    got = {}
+    for name, traverse in (("walk", api.TRAVERSE_SKIP), ("divided", api.TRAVERSE_ORDERED | api.EXACT_BOX_TESTS),
+                           ("filtered", api.TRAVERSE_ORDERED)):
+        hits = ctx.buffer(4 * n)
+        api.hemisphere(ctx, scene, cb, tb, kind, SPP, 0.0, 1.5, table, ctx.buffer(4 * n), None, hits, None, 0, n, 16,
+                       traverse)
+        got[name] = hits.download(np.uint32, n)
+    job = dict(scene=scene, coords=cb, tidx=tb, texel_count=n, spp=SPP, perms=16, min_distance=0.0, max_distance=1.5,
+               samples=table, out0=ctx.buffer(4 * n), hits0=ctx.buffer(4 * n))
+    api.Batch(ctx, [job], kind).run(api.TRAVERSE_ORDERED | api.EXACT_BOX_TESTS)
+    got["batch"] = job["hits0"].download(np.uint32, n)
+    ctx.check()
+    assert not np.array_equal(got["filtered"], got["walk"])  # the mesh shows the difference
+    assert np.array_equal(got["divided"], got["walk"]) and np.array_equal(got["batch"], got["walk"])
