@@ -65,7 +65,9 @@ __device__ __forceinline__ float gelu(float z, float& dz) {
 }
 
 // Two at once: the products and sums as packed pairs (the same roundings, half
-// the instructions), tanhf for each.
+// the instructions), tanhf for each.  The one sum that follows a product is two
+// scalar ones: packed, the two become a fused multiply-add whatever rounding
+// they name, which flips a bf16 rounding of a few activations in ten million.
 __device__ __forceinline__ uint64_t pair(float a, float b) {
   return (uint64_t)__float_as_uint(b) << 32 | __float_as_uint(a);
 }
@@ -81,7 +83,10 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
 }
 __device__ __forceinline__ float2 gelu_pair(uint64_t z) {
   const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  const uint64_t u = mul2(pair(k0, k0), add2(z, mul2(pair(k1, k1), mul2(mul2(z, z), z))));
+  const uint64_t c = mul2(pair(k1, k1), mul2(mul2(z, z), z));
+  const uint64_t s = pair(__uint_as_float((uint32_t)z) + __uint_as_float((uint32_t)c),
+                          __uint_as_float((uint32_t)(z >> 32)) + __uint_as_float((uint32_t)(c >> 32)));
+  const uint64_t u = mul2(pair(k0, k0), s);
   const uint64_t th = pair(tanhf(__uint_as_float((uint32_t)u)), tanhf(__uint_as_float((uint32_t)(u >> 32))));
   const uint64_t g = mul2(mul2(pair(0.5f, 0.5f), z), add2(pair(1.0f, 1.0f), th));
   return make_float2(__uint_as_float((uint32_t)g), __uint_as_float((uint32_t)(g >> 32)));

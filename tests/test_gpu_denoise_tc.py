@@ -114,3 +114,21 @@ def test_apply_against_forward_on_the_same_rows(ctx):
     close(out_ao.download(np.float32, n), np.clip(ao + y[:, 0], 0, 1))
     v = bn + y[:, 1:]
     close(out_bn.download(np.float32, (n, 3)), v / np.linalg.norm(v, axis=1, keepdims=True))
+
+
+def test_engines_round_alike_on_the_same_rows(ctx):
+    """Both engines add the same products in FP32 steps of 16 and apply the same
+    GELU operation for operation, so on given rows their outputs are the same
+    bits; a fused multiply-add in one GELU shows in 7 of these rows."""
+    rng = np.random.default_rng(1)
+    n = 1 << 17
+    x = np.zeros((n, 256), np.float32)
+    x[:, :250] = rng.normal(0, 0.7, (n, 250))
+    rows = ctx.upload((x.view(np.uint32) >> 16).astype(np.uint16))
+    dn = api.Denoiser(ctx, D.init_params(3))
+    got = []
+    for engine in (api.DN_ENGINE_TCGEN05, api.DN_ENGINE_MMA_SYNC):
+        dn.set_engine(engine)
+        got.append(dn.forward(rows, n).download(np.uint32, (n, 4)))
+    ctx.check()
+    assert np.array_equal(*got)
